@@ -344,9 +344,9 @@ typedef struct {
 enum { UBOLT_SWEEP_AUTO = 0, UBOLT_SWEEP_TASKS = 1, UBOLT_SWEEP_WAVE = 2 };
 
 /* Build the sweep plan: patches of patch_size consecutive cells (0 picks 64,
- * or 24 on tetrahedra;
+ * or 48 on tetrahedra;
  * at most 256), per-ordinate upwind orders, task list; then reserve the
- * factor stores (see ubolt_sweep_set_factor_limit). Host work, one upload
+ * factor stores and one scratch vector (see ubolt_sweep_set_factor_limit). Host work, one upload
  * and the sweep's only device allocations; independent of the group.
  * Called by the first sweep if not before. The streaming stage of the preconditioner, in place of
  * PCAIR (src/transport_solverk.kokkos.cxx:238-260, composite index 1). */
@@ -383,7 +383,9 @@ int ubolt_sweep_iso_f32(ubolt_ctx *ctx, const double *phi, const float *u, float
  * built, or now by this call - never inside a sweep. bytes < 0 (the
  * default): each store that fits half the free device memory at that
  * moment (at most 96 GiB), FP32 first; 0: none; otherwise the byte limit
- * for both together. Either way the result is the same, bit for bit. */
+ * for both together. What the stores leave of it may hold one scratch vector
+ * (n_rows doubles), through which a sweep between row vectors runs
+ * ordinate-major. Either way the result is the same, bit for bit. */
 int ubolt_sweep_set_factor_limit(ubolt_ctx *ctx, int64_t bytes);
 /* Plan statistics and the sticky timeout flag (synchronises `stream`):
  * returns UBOLT_ERR_TIMEOUT, and clears the flag, if a wait gave up. */

@@ -121,6 +121,51 @@ __device__ __forceinline__ void CpAsyncCommit() { asm volatile("cp.async.commit_
 template <int N>
 __device__ __forceinline__ void CpAsyncWaitGroup() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+__device__ __forceinline__ uint32_t SmemAddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void MbarInit(uint64_t *bar, uint32_t count)
+{
+   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(SmemAddr(bar)), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void MbarInitFence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+
+__device__ __forceinline__ void MbarExpectTx(uint64_t *bar, uint32_t bytes)
+{
+   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(SmemAddr(bar)), "r"(bytes) : "memory");
+}
+
+// One contiguous global -> shared copy completing on `bar` (both addresses
+// 16-byte aligned, bytes a multiple of 16)
+__device__ __forceinline__ void BulkLoad(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
+{
+   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                    SmemAddr(dst)),
+                "l"(src), "r"(bytes), "r"(SmemAddr(bar))
+                : "memory");
+}
+
+__device__ __forceinline__ bool MbarTryWait(uint64_t *bar, uint32_t parity)
+{
+   uint32_t ok;
+   asm volatile(
+       "{\n\t.reg .pred p;\n\t"
+       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+       "selp.u32 %0, 1, 0, p;\n\t}"
+       : "=r"(ok)
+       : "r"(SmemAddr(bar)), "r"(parity)
+       : "memory");
+   return ok != 0;
+}
+
+// At most limit + 1 polls of the phase
+__device__ __forceinline__ bool MbarWaitBounded(uint64_t *bar, uint32_t parity, uint32_t limit)
+{
+   for (uint32_t k = 0; k <= limit; k++)
+      if (MbarTryWait(bar, parity)) return true;
+   return false;
+}
+
 template <typename T>
 __device__ __forceinline__ T Dot3(const T *__restrict__ om, const T *__restrict__ n)
 {
@@ -350,11 +395,11 @@ __host__ inline int CellsPerBlock(int A)
 
 // The factors of one (cell, ordinate) for the sweep: W = B^{-1} of its
 // streaming + removal block, and G_s = W (s_f face_up_f) for each gathered
-// face f in face order (slot s); element (s, ii, j) goes to Gout[s * gs + (ii * NB + j) * ge].
+// face f in face order (slot s); element (s, ii, j) goes to Gout[s * gs + ii * gr + j * gj].
 // A singular block gives zero factors. Returns false then.
 template <typename T, int NB, int F>
 __device__ __forceinline__ bool CellFactors(const DevGeom<T> &g, int64_t c, const T om[3], uint32_t mask, T W[NB][NB],
-                                            T *Gout, size_t gs, size_t ge)
+                                            T *Gout, size_t gs, size_t gr, size_t gj)
 {
    const int32_t cl = g.cls[c];
    T B[NB][NB];
@@ -387,7 +432,7 @@ __device__ __forceinline__ bool CellFactors(const DevGeom<T> &g, int64_t c, cons
                T u = T(0);
 #pragma unroll
                for (int kk = 0; kk < NB; kk++) u += W[ii][kk] * Ms[kk][j];
-               Gf[(size_t)(ii * NB + j) * ge] = u;
+               Gf[(size_t)ii * gr + (size_t)j * gj] = u;
             }
       }
       slot++;

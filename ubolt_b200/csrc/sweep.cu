@@ -20,19 +20,33 @@
 // upstream tasks are still walking: the chain of dependencies runs cell to
 // cell through L2 with no flags, fences or task-granular barriers.
 //
-// Everything off that chain happens first, in a prologue: the lanes build and
-// invert every cell's nb x nb block from geometry and sigma_t, and keep
-// y0 = B^{-1} q and G_f = B^{-1} s_f face_up_f (one per gathered face) in the
-// warp's shared-memory slice. The walk then runs level by level, touching
-// shared memory for in-task neighbours: psi_c = y0 - sum_f G_f psi(up_f).
+// Everything off that chain happens first, in a prologue: y0 = B^{-1} q and
+// the couplings G_f = B^{-1} s_f face_up_f (one per gathered face) of every
+// cell of the task go into the warp's shared-memory slice. The walk then runs
+// level by level over a table of values in shared memory - the task's own
+// cells and its ghosts, the cells of earlier tasks it reads: psi_c = y0 -
+// sum_f G_f psi(up_f), one lane per row of a cell.
 // Deadlock-free: a task polls only values of lower-numbered tasks, which were
 // taken by warps already running. Every poll is bounded; a poll that gives up
 // records a timeout, reads the value as zero and the sweep completes.
+//
+// What bounds it: the latency of the tasks and of the upwind chain, not bytes
+// or flops (256^2 triangles, DG1, S8, FP64: 154 thousand tasks of 34 cells in 15
+// levels). So the walk is built for few instructions and no divergence per
+// level (a warp that splits on a branch loses about 100 cycles, as much as a
+// level's arithmetic), and a wait asks for what the next levels wait for as
+// well. Per sweep with an isotropic source and psi ordinate-major, before (a
+// lane per cell, each level polling for itself) and now, FP64 / FP32: 256^2
+// triangles 942 / 791 -> 595 / 486 us, 200^2 quadrilaterals 635 / 555 -> 316 /
+// 267, 20^3 cubes of Kuhn tetrahedra 1447 / 1159 -> 982 / 678, 40^3 hexahedra
+// 1186 / 684 -> 593 / 402.
 #include "ctx.h"
 #include "sweep_plan.h"
 #include "wave.h"
 
 #include <algorithm>
+#include <cstring>
+#include <type_traits>
 #include <vector>
 
 // The task counter and the error words sit on separate 128-byte lines: every
@@ -40,19 +54,25 @@
 // Words [kCtrlNever, kCtrlNever + 2) hold a sentinel nothing overwrites (the
 // target of the bounded-wait test hook).
 constexpr int kCtrlCounter = 0, kCtrlError = ubolt::kSweepCtrlError, kCtrlNever = 48, kCtrlWords = 64;
-constexpr int kSweepBlocksPerSm = 8;  // of 4 warps
+constexpr int kSweepWarpsPerSm = 32;
+constexpr size_t kViaBytes = (size_t)8 << 20;
+constexpr uint32_t kCopyTries = 1u << 22;  // bounded wait for a task's bulk copy
 constexpr int kDefaultPatch = 64;
 
 // The default patch: half a tile of the mesh builders' cell numbering (8 x 8
-// quads, 4^3 hexes), and four cubes' worth of Kuhn tetrahedra. Measured per
-// isotropic-source sweep at S8 (FP64 / FP32): 256^2 triangles 0.89 / 0.78 ms
-// at 64 cells against 0.97 / 0.83 at 32; 44^3 Kuhn tets 15.3 / 12.0 ms at 24
-// against 18.2 / 14.1 at 32 and 23.4 / 15.8 at 64. On the 128^3 hex box 64
-// stays: the 4-group FP64 solve, whose factors are built in the sweep, took
-// 1.64 s at 64 against 1.79 s at 32 (the mixed solve 1.08 / 1.07 s)
+// quads, 4^3 hexes), and eight cubes' worth of Kuhn tetrahedra. Measured per
+// isotropic-source sweep at S8 (FP64 / FP32, us): 256^2 triangles 595 / 488 at
+// 64 cells, 607 / 418 at 128, 921 / 813 at 32; 200^2 quadrilaterals 301 / 268
+// at 64, 354 / 312 at 32, 312 / 263 at 128; 20^3 cubes of Kuhn tetrahedra 901 /
+// 492 at 48, 946 / 673 at 24, 1361 / 599 at 96; 40^3 hexahedra 603 / 399 at 64,
+// 683 / 350 at 32
 static int DefaultPatch(const ubolt_ctx *ctx)
 {
-   return (ctx->dim == 3 && ctx->F == 4) ? 24 : kDefaultPatch;
+   return (ctx->dim == 3 && ctx->F == 4) ? 48 : kDefaultPatch;
+}
+
+namespace ubolt {
+struct Task;
 }
 
 struct ubolt_sweep_plan {
@@ -60,24 +80,24 @@ struct ubolt_sweep_plan {
    int64_t n_tasks = 0, n_lagged = 0, n_split = 0, total_levels = 0;
    int32_t max_levels = 0, max_inflow = 0;
    // Device arrays (owned by the context's allocation list)
-   const int32_t *task_pa = nullptr;    // [n_tasks] patch * A + ordinate
+   const ubolt::Task *task = nullptr;   // [n_tasks]
    const int32_t *dep_ptr = nullptr;    // [n_tasks + 1]
    const int32_t *deps = nullptr;       // upstream task ids
-   const int64_t *cell_ptr = nullptr;   // [n_tasks + 1]
-   const uint8_t *tcell = nullptr;      // local cell index in the patch, level order
+   const uint16_t *sched = nullptr;     // per entry, SchedWords(F) words: the local cell, then per gathered face the
+                                        // upwind cell's place in the task's value table (see SweepDev)
    const uint16_t *tmask = nullptr;     // upwind faces: in task (bit f) / earlier task (bit 8 + f)
-   const int32_t *lvl_ptr = nullptr;    // [n_tasks + 1]
-   const uint16_t *lvl = nullptr;       // level end positions within the task
-   const uint16_t *tlev = nullptr;      // [entries] level of each entry within its task
-   const int32_t *tlink = nullptr;      // [entries][slots] upwind link per gathered face: >= 0 the cell in an
-                                        // earlier task, -2 - local for a cell of this task, -1 none
+   const uint16_t *pass = nullptr;      // end positions of every task's passes (levels cut at 32 / nb positions)
+   const int32_t *ghost = nullptr;      // the cells of earlier tasks each task reads
+   int n_loc = 0;                       // most (positions + ghosts) of a task, plus one
+   int n_ghost = 1;                     // most ghosts of a task
    uint32_t *ctrl = nullptr;            // [kCtrlCounter] task counter; [kCtrlError] error flag, [kCtrlError + 1] timeout count
-   int grid = 0, warps_per_block = 4, slots = 1;
+   int grid = 0, slots = 1;
    uint32_t spin_limit = 1u << 22;
    int64_t unmet_task = -1;  // ubolt_sweep_test_wait: one task polls a value nothing writes
    // The factor store (B^{-1} and couplings per task entry) per precision,
    // valid for the group epoch it was built in; limit < 0: automatic
    void *fac[2] = {nullptr, nullptr};
+   void *scratch = nullptr;  // one FP64 vector: a sweep between row vectors runs ordinate-major in it
    uint64_t fac_epoch[2] = {0, 0};
    int64_t fac_limit = -1;
    // The wave plan (one block per ordinate), where every ordinate's upwind
@@ -94,7 +114,7 @@ struct ubolt_sweep_plan {
    int64_t unmet_level = -1;  // ubolt_sweep_test_wait: one level's copy is never issued
    ~ubolt_sweep_plan()
    {
-      for (void *f : fac)
+      for (void *f : {fac[0], fac[1], scratch})
          if (f) cudaFree(f);
    }
 };
@@ -130,14 +150,85 @@ __device__ __forceinline__ float LoadRelaxed(const float *p)
    asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
    return v;
 }
-__device__ __forceinline__ void StoreRelaxed(double *p, double v)
+// Stores of psi, and the sweep's other one-lane operations, under a
+// predicate instead of a branch (a branch that splits the warp costs about
+// 100 cycles)
+__device__ __forceinline__ void StoreRelaxedIf(bool yes, double *p, double v)
 {
-   asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.relaxed.gpu.global.f64 [%0], %1;\n\t}" ::"l"(p),
+                "d"(v), "r"((int)yes)
+                : "memory");
 }
-__device__ __forceinline__ void StoreRelaxed(float *p, float v)
+__device__ __forceinline__ void StoreRelaxedIf(bool yes, float *p, float v)
 {
-   asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.relaxed.gpu.global.f32 [%0], %1;\n\t}" ::"l"(p),
+                "f"(v), "r"((int)yes)
+                : "memory");
 }
+__device__ __forceinline__ void LoadRelaxedIf(bool yes, const double *p, double &v)
+{
+   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.relaxed.gpu.global.f64 %0, [%1];\n\t}"
+                : "+d"(v)
+                : "l"(p), "r"((int)yes)
+                : "memory");
+}
+__device__ __forceinline__ void LoadRelaxedIf(bool yes, const float *p, float &v)
+{
+   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.relaxed.gpu.global.f32 %0, [%1];\n\t}"
+                : "+f"(v)
+                : "l"(p), "r"((int)yes)
+                : "memory");
+}
+__device__ __forceinline__ void StoreSharedIf(bool yes, double *p, double v)
+{
+   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.shared.f64 [%0], %1;\n\t}" ::"r"(SmemAddr(p)),
+                "d"(v), "r"((int)yes)
+                : "memory");
+}
+__device__ __forceinline__ void StoreSharedIf(bool yes, float *p, float v)
+{
+   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.shared.f32 [%0], %1;\n\t}" ::"r"(SmemAddr(p)),
+                "f"(v), "r"((int)yes)
+                : "memory");
+}
+__device__ __forceinline__ uint32_t AtomicIncIf(bool yes, uint32_t *p)
+{
+   uint32_t v = 0;
+   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p atom.global.add.u32 %0, [%1], 1;\n\t}"
+                : "+r"(v)
+                : "l"(p), "r"((int)yes)
+                : "memory");
+   return v;
+}
+// mbarrier.arrive.expect_tx, then one bulk copy with an L2 policy completing on it
+__device__ __forceinline__ void BulkLoadIf(bool yes, void *dst, const void *src, uint32_t bytes, uint64_t *bar,
+                                           uint64_t policy)
+{
+   asm volatile(
+       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+       "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %2;\n\t"
+       "@p cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+       "\n\t}" ::"r"(SmemAddr(dst)),
+       "l"(src), "r"(bytes), "r"(SmemAddr(bar)), "l"(policy), "r"((int)yes)
+       : "memory");
+}
+// N values from shared memory, as 16-byte words where they are aligned so
+template <typename T, int N, bool WIDE>
+__device__ __forceinline__ void LoadRow(const T *p, T (&v)[N])
+{
+   if constexpr (WIDE) {
+#pragma unroll
+      for (int u = 0; u < N * (int)sizeof(T) / 16; u++) {
+         const int4 w = reinterpret_cast<const int4 *>(p)[u];
+         memcpy(reinterpret_cast<char *>(v) + 16 * u, &w, 16);
+      }
+   } else {
+#pragma unroll
+      for (int e = 0; e < N; e++) v[e] = p[e];
+   }
+}
+__device__ __forceinline__ uint32_t TopWord(double v) { return (uint32_t)__double2hiint(v); }
+__device__ __forceinline__ uint32_t TopWord(float v) { return (uint32_t)__float_as_int(v); }
 __device__ __forceinline__ bool IsSentinel(double v) { return __double_as_longlong(v) == -1LL; }
 __device__ __forceinline__ bool IsSentinel(float v) { return __float_as_int(v) == -1; }
 template <typename T>
@@ -151,17 +242,42 @@ __device__ __forceinline__ float Sentinel<float>() { return __int_as_float(-1); 
 __device__ __forceinline__ double Publishable(double v) { return IsSentinel(v) ? __longlong_as_double(0x7ff8000000000001LL) : v; }
 __device__ __forceinline__ float Publishable(float v) { return IsSentinel(v) ? __int_as_float(0x7fc00001) : v; }
 
+// Words of an entry's schedule record: the local cell and up to F - 1 links
+__host__ __device__ constexpr int SchedWords(int F) { return F <= 4 ? 4 : 8; }
+
+// A task as one 32-byte record: cells, passes and ghosts in the first word,
+// the patch, its first entry, first ghost and first pass, the ordinate
+struct __align__(16) Task {
+   uint32_t counts;
+   int32_t patch;
+   int64_t off;
+   int64_t ghost0;
+   int32_t pass0, ordinate;
+   __host__ __device__ int ncell() const { return counts & 1023; }
+   __host__ __device__ int npass() const { return (counts >> 10) & 1023; }
+   __host__ __device__ int nghost() const { return (int)(counts >> 20); }
+};
+__device__ __forceinline__ Task LoadTask(const Task *p)
+{
+   Task t;
+   const int4 *s = reinterpret_cast<const int4 *>(p);
+   const int4 a = __ldg(s), b = __ldg(s + 1);
+   memcpy(&t, &a, 16);
+   memcpy(reinterpret_cast<char *>(&t) + 16, &b, 16);
+   return t;
+}
+
 struct SweepDev {
    int32_t P, A;
    int64_t n_tasks;
-   const int32_t *task_pa;
-   const int64_t *cell_ptr;
-   const uint8_t *tcell;
-   const uint16_t *tmask;
-   const uint16_t *tlev;
-   const int32_t *tlink;
-   const int32_t *lvl_ptr;
-   const uint16_t *lvl;
+   const Task *task;        // [n_tasks]
+   const uint16_t *sched;   // per entry, SchedWords(F) words: the local cell, then per gathered face the upwind cell's
+                            // place in the task's value table, in elements - nb times 1 + its position, or 1 + ncell +
+                            // its place among the task's ghosts, or 0 (a zero: no such face)
+   const uint16_t *tmask;   // [entries] gathered faces (factors built in the sweep, and the store)
+   const int32_t *ghost;    // per task, the cells of earlier tasks it reads
+   int32_t n_loc, n_ghost;
+   const uint16_t *pass;    // end position of every pass of every task
    uint32_t *ctrl;
    uint32_t spin_limit;
    int32_t slots;
@@ -177,374 +293,426 @@ struct SweepDev {
    // (NB A, A, 1), or ordinate-major (NB, 1, n_cells NB), where a task's
    // cells of one ordinate are contiguous and it writes whole sectors
    int64_t os_c, os_j, os_a;
+   // q(c, j, a) at q[c qs_c + j qs_j + a qs_a], the same two layouts
+   int64_t qs_c, qs_j, qs_a;
 };
 
 // Per-warp shared-memory slice, for P cells and S gathered faces per cell
-// Each nb x nb coupling in shared memory takes a 16-byte multiple, so the
-// walk reads it with 16-byte loads
-__host__ __device__ constexpr int GStride(int NB, int elem) { return (NB * NB * elem + 15) / 16 * 16 / elem; }
-
-// A position's S couplings in shared memory. A run of a multiple of four
-// 16-byte units (the 4 x 4 blocks of 3D DG1) is padded by one unit: a
-// quarter-warp's 16-byte reads of one slot at consecutive positions would
-// otherwise fall on the same banks, 8-way. Shorter conflicts are left alone:
-// the padding's shared memory costs L1 (the shapes on triangles and quads
-// run slower with it).
-__host__ __device__ constexpr int PosStride(int S, int NB, int elem)
-{
-   return (S * GStride(NB, elem) * elem / 16 % 4 == 0 ? S * GStride(NB, elem) * elem + 16
-                                                       : S * GStride(NB, elem) * elem) / elem;
-}
+// The stride between positions, in elements, where lanes write their own
+// position's gc couplings into shared memory: a multiple of 64 bytes would put
+// every lane on the same banks (the 4 x 4 blocks of 3D DG1), so one 16-byte
+// unit is added there
+__host__ __device__ constexpr int LaneStride(int gc, int elem) { return gc * elem % 64 == 0 ? gc + 16 / elem : gc; }
 
 struct SweepSlice {
-   size_t loc, G, bytes;
-   __host__ __device__ SweepSlice(int P, int S, int NB, int elem)
+   int loc, G, rec, pass, ghost, bar, bytes;
+   __host__ __device__ constexpr SweepSlice(int P, int S, int F, int NB, int n_loc, int n_ghost, int elem, bool cached)
+       : loc(0), G(0), rec(0), pass(0), ghost(0), bar(0), bytes(0)
    {
-      auto up = [](size_t v) { return (v + 15) & ~(size_t)15; };
-      loc = 0;                                           // T [P][NB], by local cell
-      G = up(loc + (size_t)P * NB * elem);               // T [P][PosStride], by position
-      bytes = up(G + (size_t)P * PosStride(S, NB, elem) * elem);
+      G = 16;                                                     // after the copy's mbarrier: T [ncell][NB][S][NB],
+                                                                  // and up to one 16-byte unit of lead-in
+      loc = G + Pad16(P * (cached ? S * NB * NB : LaneStride(S * NB * NB, elem)) * elem, 1) + 16;
+                                                                  // T [n_loc][NB]: a zero, the positions, the ghosts
+      rec = Pad16(loc + n_loc * NB * elem, 1);                    // uint16 [P][SchedWords(F)]
+      ghost = rec + P * SchedWords(F) * 2;                        // int32 [n_ghost]: the ghosts' cells
+      pass = ghost + n_ghost * 4;                                 // uint16 [P + 2]
+      bytes = Pad16(pass + (P + 2) * 2, 1);
    }
 };
 
-// The NB values psi(up, :, a) of an upwind cell in an earlier task, polled
-// until its task has stored them all. Bounded: on giving up the sticky error
-// flag is set, the timeout counted, and the missing values read as zero.
+
+// The factor store, per task from element off R, R = NB^2 (1 + S): W = B^{-1}
+// element-major over the task's positions (element e of position i at
+// e ncell + i, the lanes of a prologue read consecutive words), then the
+// couplings position by position, row-major over (row, slot, column): what one
+// lane of the walk reads is one run. Unused slots are zero. Independent of the
+// right-hand side: built once per group, read by every sweep. The couplings
+// are laid out in shared memory and written 32 positions at a time.
+// Slots from..S of a position's couplings set to zero
 template <typename T, int NB>
-__device__ __forceinline__ void PollUpwind(const T *p, int stride, const SweepDev &s, T xn[NB])
+__device__ __forceinline__ void ZeroSlots(T *G, int from, int S)
 {
-   bool missing = false;
+   for (int sl = from; sl < S; sl++)
 #pragma unroll
-   for (int j = 0; j < NB; j++) {
-      xn[j] = LoadRelaxed(p + (size_t)j * stride);
-      missing |= IsSentinel(xn[j]);
-   }
-   uint32_t spins = 0;
-   while (missing) {
-      // The sticky error flag (another wait gave up) is read once per 1024
-      // spins, so that waiting lanes stay off its line
-      if (++spins > s.spin_limit || ((spins & 1023u) == 0 && *(volatile uint32_t *)&s.ctrl[kCtrlError])) {
-         atomicOr(&s.ctrl[kCtrlError], 1u);
-         atomicAdd(&s.ctrl[kCtrlError + 1], 1u);
-#pragma unroll
-         for (int j = 0; j < NB; j++)
-            if (IsSentinel(xn[j])) xn[j] = T(0);
-         return;
-      }
-      if (spins > 32) __nanosleep(spins < 4096 ? 32 : 256);
-      missing = false;
-#pragma unroll
-      for (int j = 0; j < NB; j++)
-         if (IsSentinel(xn[j])) {
-            xn[j] = LoadRelaxed(p + (size_t)j * stride);
-            missing |= IsSentinel(xn[j]);
-         }
-   }
+      for (int e = 0; e < NB * NB; e++) G[(e / NB) * S * NB + sl * NB + e % NB] = T(0);
 }
 
-// y -= G x for one nb x nb coupling held in shared memory (16-byte aligned,
-// GStride elements), read with 16-byte loads
-template <typename T, int NB>
-__device__ __forceinline__ void SubCoupling(const T *__restrict__ Gf, const T xn[NB], T y[NB])
-{
-   constexpr int GS = GStride(NB, (int)sizeof(T));
-   constexpr int PER = 16 / (int)sizeof(T);
-   T gv[GS];
-#pragma unroll
-   for (int v = 0; v < GS / PER; v++) {
-      if constexpr (sizeof(T) == 8) {
-         const double2 d = reinterpret_cast<const double2 *>(Gf)[v];
-         gv[2 * v] = d.x;
-         gv[2 * v + 1] = d.y;
-      } else {
-         const float4 d = reinterpret_cast<const float4 *>(Gf)[v];
-         gv[4 * v] = d.x;
-         gv[4 * v + 1] = d.y;
-         gv[4 * v + 2] = d.z;
-         gv[4 * v + 3] = d.w;
-      }
-   }
-#pragma unroll
-   for (int ii = 0; ii < NB; ii++) {
-      T u = T(0);
-#pragma unroll
-      for (int j = 0; j < NB; j++) u += gv[ii * NB + j] * xn[j];
-      y[ii] -= u;
-   }
-}
-
-// The factor store: per task, element-major over its positions, so a warp's
-// lanes read consecutive words - element r of position i of task t at
-// cell_ptr[t] R + r ncell_t + i, R = NB^2 (1 + S): W, then G_0 .. G_{S-1}.
-// Independent of the right-hand side: built once per group, read by every sweep.
 template <typename T, int NB, int F>
 __global__ void __launch_bounds__(128) FactorKernel(const DevGeom<T> g, const SweepDev s, T *__restrict__ fac)
 {
+   extern __shared__ __align__(16) unsigned char smem_raw[];
    const int lane = threadIdx.x & 31;
    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
    const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-   const int S = s.slots;
+   const int S = s.slots, GC = S * NB * NB;
+   const int GP = LaneStride(GC, (int)sizeof(T));
+   T *stage = reinterpret_cast<T *>(smem_raw) + (size_t)(threadIdx.x >> 5) * 32 * GP;
+   const unsigned magic = ((1u << 20) + GC - 1) / GC;  // e / GC for e < 32 GC, GC <= 80 (exact: e * GC < 2^20)
    const size_t R = (size_t)NB * NB * (1 + S);
    for (int64_t t = warp; t < s.n_tasks; t += n_warps) {
-      const int32_t pa = s.task_pa[t];
-      const int64_t off = s.cell_ptr[t];
-      const int ncell = (int)(s.cell_ptr[t + 1] - off);
-      const int32_t p = pa / s.A;
-      const int a = pa - p * s.A;
-      const int64_t base = (int64_t)p * s.P;
+      const Task tk = LoadTask(s.task + t);
+      const int ncell = tk.ncell();
+      const int a = tk.ordinate;
+      const int64_t base = (int64_t)tk.patch * s.P;
       const T om[3] = {g.omega[3 * a], g.omega[3 * a + 1], g.omega[3 * a + 2]};
-      T *ft = fac + (size_t)off * R;
-      for (int i = lane; i < ncell; i += 32) {
-         T W[NB][NB];
-         CellFactors<T, NB, F>(g, base + s.tcell[off + i], om, s.tmask[off + i], W, ft + (size_t)NB * NB * ncell + i,
-                               (size_t)NB * NB * ncell, (size_t)ncell);
-#pragma unroll
-         for (int ii = 0; ii < NB; ii++)
-#pragma unroll
-            for (int j = 0; j < NB; j++) ft[(size_t)(ii * NB + j) * ncell + i] = W[ii][j];
-      }
-   }
-}
-
-// PL: positions per lane, P <= 32 PL. Lane l owns positions l, l + 32, ...;
-// its cells' schedule (local index, level, upwind links) stays in registers.
-// CACHED: the factors come from the store, else they are computed here.
-// Resident blocks of 4 warps the compiler should fit per SM: the sweep is
-// bound by per-task latency, and FP64 nb <= 3 with one cell per lane fits a
-// fifth block without spilling (with two, the spills cost more than the
-// block). On triangles with two cells per lane FP64 keeps a fourth block
-// (at most 128 registers, no spill): left free it took 134 and three
-// blocks, and the 256^2 triangle sweep 0.969 ms against 0.941
-template <typename T, int NB, int F, int PL>
-constexpr int SweepMinBlocks()
-{
-   return (sizeof(T) == 8 && NB <= 3 && PL == 1) ? 5 : (sizeof(T) == 8 && NB <= 3 && F == 3 && PL == 2) ? 4 : 1;
-}
-
-template <typename T, int NB, int F, int PL, bool CACHED>
-__global__ void __launch_bounds__(128, SweepMinBlocks<T, NB, F, PL>()) SweepKernel(const DevGeom<T> g, const SweepDev s, const T *__restrict__ q,
-                                                   T *__restrict__ psi, const T *__restrict__ fac)
-{
-   extern __shared__ __align__(16) unsigned char smem_raw[];
-   const int lane = threadIdx.x & 31;
-   const int warp = threadIdx.x >> 5;
-   const int S = s.slots;     // coupling matrices kept per cell
-   constexpr int SM = F - 1;  // most gathered faces of a cell
-   const SweepSlice L(s.P, S, NB, (int)sizeof(T));
-   unsigned char *slice = smem_raw + (size_t)warp * L.bytes;
-   T *loc = reinterpret_cast<T *>(slice + L.loc);
-   T *G = reinterpret_cast<T *>(slice + L.G);
-   const int A = s.A;
-   const T *never = reinterpret_cast<const T *>(s.ctrl + kCtrlNever);
-   const size_t R = (size_t)NB * NB * (1 + S);
-   constexpr int GS = GStride(NB, (int)sizeof(T));
-   const int PS = PosStride(S, NB, (int)sizeof(T));
-   // The factor store is read once per sweep: its lines go first from L2, so
-   // that they do not push out psi and the schedule other warps are reading
-   const uint64_t stream_once = EvictFirstPolicy();
-   // The task's five scalars, one lane each, in one round trip
-   auto scalars = [&](int64_t tt) -> int64_t {
-      if (tt >= s.n_tasks) return 0;
-      if (lane == 0) return s.task_pa[tt];
-      if (lane == 1) return s.cell_ptr[tt];
-      if (lane == 2) return s.cell_ptr[tt + 1];
-      if (lane == 3) return s.lvl_ptr[tt];
-      if (lane == 4) return s.lvl_ptr[tt + 1];
-      return 0;
-   };
-   for (;;) {
-      // A task is claimed only when the warp is free: a task claimed while
-      // the warp still walks (and waits in) another would sit idle behind it,
-      // and the tasks downstream of it would wait too (claiming even two
-      // levels before the walk ends measured slower)
-      int64_t t = 0;
-      if (lane == 0) t = (int64_t)atomicAdd(&s.ctrl[kCtrlCounter], 1u);
-      t = __shfl_sync(0xffffffffu, t, 0);
-      if (t >= s.n_tasks) break;
-      const int64_t v = scalars(t);
-      const int32_t pa = (int32_t)__shfl_sync(0xffffffffu, v, 0);
-      const int64_t off = __shfl_sync(0xffffffffu, v, 1);
-      const int ncell = (int)(__shfl_sync(0xffffffffu, v, 2) - off);
-      const int32_t l0 = (int32_t)__shfl_sync(0xffffffffu, v, 3);
-      const int nlev = (int)(__shfl_sync(0xffffffffu, v, 4) - l0);
-      const int32_t p = pa / A;
-      const int a = pa - p * A;
-      const int64_t base = (int64_t)p * s.P;
-
-      // Prologue - nothing here depends on upstream values: loc gets
-      // y0 = B^{-1} q, G the couplings of the gathered faces, and each lane
-      // its positions' schedule
-      int my_local[PL], my_lev[PL], my_ul[PL][SM];
-      int32_t my_up[PL][SM];
-      // The schedule, and with the store every factor load of every owned
-      // position, issued before any is used (the couplings straight into
-      // shared memory by cp.async); with the links in hand, the upwind values
-      // of earlier tasks are loaded in the same round as q
-      constexpr bool kPreloadW = CACHED && PL <= 2;  // more positions: loaded where used
-      constexpr bool kPrefetch = PL <= 2;
-      T W[kPreloadW ? PL : 1][NB][NB];
-      T xp[kPrefetch ? PL : 1][SM][NB];
-      const bool hook = (t == s.unmet_task);
-#pragma unroll
-      for (int k = 0; k < PL; k++) {
-         const int i = lane + 32 * k;
-         const bool valid = i < ncell;
-         my_local[k] = valid ? s.tcell[off + i] : 0;
-         my_lev[k] = valid ? s.tlev[off + i] : -1;
-#pragma unroll
-         for (int sl = 0; sl < SM; sl++) {
-            const int32_t lk = (valid && sl < S) ? s.tlink[(off + i) * S + sl] : -1;
-            my_up[k][sl] = lk >= 0 ? lk : -1;
-            my_ul[k][sl] = lk <= -2 ? -2 - lk : -1;
-         }
-         if constexpr (CACHED) {
-            if (valid) {
-               const T *ft = fac + (size_t)off * R + i;
-               if constexpr (kPreloadW) {
-#pragma unroll
-                  for (int ii = 0; ii < NB; ii++)
-#pragma unroll
-                     for (int j = 0; j < NB; j++) W[k][ii][j] = LoadHint(ft + (size_t)(ii * NB + j) * ncell, stream_once);
-               }
-#pragma unroll
-               for (int e = 0; e < SM * NB * NB; e++)
-                  if (e < S * NB * NB)
-                     CpAsyncHint<sizeof(T)>(G + (size_t)i * PS + (e / (NB * NB)) * GS + e % (NB * NB),
-                                            ft + (size_t)(NB * NB + e) * ncell, stream_once);
-            }
-         }
-         if constexpr (kPrefetch) {
-#pragma unroll
-            for (int sl = 0; sl < SM; sl++)
-#pragma unroll
-               for (int j = 0; j < NB; j++)
-                  xp[k][sl][j] = (my_up[k][sl] >= 0 && !hook)
-                                    ? LoadRelaxed(psi + (int64_t)my_up[k][sl] * s.os_c + j * s.os_j + a * s.os_a)
-                                    : Sentinel<T>();
-         }
-      }
-#pragma unroll
-      for (int k = 0; k < PL; k++) {
-         const int i = lane + 32 * k;
-         if (i >= ncell) continue;
-         const int local = my_local[k];
-         const int64_t c = base + local;
-         T r[NB];
-         if (s.aff_phi) {
-            const double al = s.aff_iso ? 0.0 : *s.aff_alpha;
-            const double ua = s.aff_u ? (double)static_cast<const T *>(s.aff_u)[a] : 1.0;
-#pragma unroll
-            for (int j = 0; j < NB; j++) {
-               const int64_t node = c * NB + j;
-               r[j] = s.aff_iso ? (T)(ua * s.aff_phi[node] / (s.aff_inv_volume ? (double)g.volume[c] : 1.0))
-                                : (T)(al * (double)q[node * A + a] + ua * (s.aff_phi[node] - al * s.aff_rho[node]));
-            }
-         } else {
-#pragma unroll
-            for (int j = 0; j < NB; j++) r[j] = q[(c * NB + j) * A + a];
-         }
-         T Wk[NB][NB];
-         if constexpr (kPreloadW) {
+      T *ft = fac + (size_t)tk.off * R;
+      for (int i0 = 0; i0 < ncell; i0 += 32) {
+         const int i = i0 + lane;
+         if (i < ncell) {
+            T W[NB][NB];
+            const uint32_t mask = s.tmask[tk.off + i];
+            T *Gi = stage + lane * GP;
+            CellFactors<T, NB, F>(g, base + s.sched[(tk.off + i) * SchedWords(F)], om, mask, W, Gi, (size_t)NB,
+                                  (size_t)S * NB, 1);
+            ZeroSlots<T, NB>(Gi, __popc((mask | (mask >> 8)) & 0xffu), S);
 #pragma unroll
             for (int ii = 0; ii < NB; ii++)
 #pragma unroll
-               for (int j = 0; j < NB; j++) Wk[ii][j] = W[k][ii][j];
-         } else if constexpr (CACHED) {
-            const T *ft = fac + (size_t)off * R + i;
-#pragma unroll
-            for (int ii = 0; ii < NB; ii++)
-#pragma unroll
-               for (int j = 0; j < NB; j++) Wk[ii][j] = ft[(size_t)(ii * NB + j) * ncell];
-         } else {
-            const T om[3] = {g.omega[3 * a], g.omega[3 * a + 1], g.omega[3 * a + 2]};
-            CellFactors<T, NB, F>(g, c, om, s.tmask[off + i], Wk, G + (size_t)i * PS, (size_t)GS, 1);
+               for (int j = 0; j < NB; j++) ft[(size_t)(ii * NB + j) * ncell + i] = W[ii][j];
          }
-         T y[NB];
-#pragma unroll
-         for (int ii = 0; ii < NB; ii++) {
-            T u = T(0);
-#pragma unroll
-            for (int j = 0; j < NB; j++) u += Wk[ii][j] * r[j];
-            y[ii] = u;
-         }
-         // A position whose upwind values from earlier tasks are all stored
-         // already has them folded in now; the others poll at their level.
-         // Either way a cell subtracts its earlier-task couplings first, in
-         // slot order, then its in-task ones: the result does not depend on
-         // timing.
-         if constexpr (kPrefetch) {
-            bool any = false, ready = true;
-#pragma unroll
-            for (int sl = 0; sl < SM; sl++) {
-               any |= my_up[k][sl] >= 0;
-#pragma unroll
-               for (int j = 0; j < NB; j++) ready &= !(my_up[k][sl] >= 0 && IsSentinel(xp[k][sl][j]));
-            }
-            if (any && ready) {
-               if constexpr (CACHED) CpAsyncWaitAll();  // this lane's couplings
-#pragma unroll
-               for (int sl = 0; sl < SM; sl++) {
-                  if (my_up[k][sl] < 0) continue;
-                  SubCoupling<T, NB>(G + (size_t)i * PS + sl * GS, xp[k][sl], y);
-                  my_up[k][sl] = -1;
-               }
-            }
-         }
-#pragma unroll
-         for (int ii = 0; ii < NB; ii++) loc[local * NB + ii] = y[ii];
-      }
-      if constexpr (CACHED) CpAsyncWaitAll();
-      __syncwarp();
-      bool hook_left = hook;
-
-      // Level by level: psi_c = y0 - sum_f G_f psi(up_f), an in-task
-      // neighbour from shared memory, an earlier task's polled from L2
-      for (int l = 0; l < nlev; l++) {
-#pragma unroll
-         for (int k = 0; k < PL; k++) {
-            if (my_lev[k] != l) continue;
-            const int i = lane + 32 * k;
-            const int local = my_local[k];
-            T y[NB];
-#pragma unroll
-            for (int j = 0; j < NB; j++) y[j] = loc[local * NB + j];
-#pragma unroll
-            for (int sl = 0; sl < SM; sl++) {
-               if (my_up[k][sl] < 0) continue;
-               const T *src = psi + (int64_t)my_up[k][sl] * s.os_c + a * s.os_a;
-               int stride = (int)s.os_j;
-               if (hook_left) {
-                  src = never;  // test hook: this wait can never be met
-                  stride = 0;
-                  hook_left = false;
-               }
-               T xn[NB];
-               PollUpwind<T, NB>(src, stride, s, xn);
-               SubCoupling<T, NB>(G + (size_t)i * PS + sl * GS, xn, y);
-            }
-#pragma unroll
-            for (int sl = 0; sl < SM; sl++) {
-               if (my_ul[k][sl] < 0) continue;
-               T xn[NB];
-#pragma unroll
-               for (int j = 0; j < NB; j++) xn[j] = loc[my_ul[k][sl] * NB + j];
-               SubCoupling<T, NB>(G + (size_t)i * PS + sl * GS, xn, y);
-            }
-            const int64_t c = base + local;
-#pragma unroll
-            for (int j = 0; j < NB; j++) {
-               loc[local * NB + j] = y[j];
-               StoreRelaxed(&psi[c * s.os_c + j * s.os_j + a * s.os_a], Publishable(y[j]));
-            }
+         __syncwarp();
+         T *Gt = ft + (size_t)NB * NB * ncell + (size_t)i0 * GC;
+         const int n = min(32, ncell - i0) * GC;
+#pragma unroll 4
+         for (int e = lane; e < n; e += 32) {
+            const int i = (int)((e * magic) >> 20);
+            Gt[e] = stage[i * GP + (e - i * GC)];
          }
          __syncwarp();
       }
    }
 }
 
+// Blocks of two warps the registers should leave room for per SM: eight (at
+// most 128 registers), ten for FP32 tetrahedra, whose small tasks are bound by
+// their number in flight (678 against 780 us per sweep of 20^3 cubes; the
+// other shapes measured the same or slower), and no cap where the blocks would
+// spill heavily and shared memory holds fewer anyway
+template <typename T, int NB, int S, int KU>
+constexpr int SweepMinBlocks()
+{
+   if (sizeof(T) == 8 && NB == 4 && (KU > 1 || S == 5)) return 1;
+   return sizeof(T) == 4 && NB == 4 && KU == 1 ? 10 : 8;
+}
+
+// The sweep. A warp takes one task at a time.
+//
+// Prologue: one record says where the task's data are; then, all in flight at
+// once, its couplings G come into shared memory by one bulk copy, and each
+// lane reads, for its positions, the schedule record, W and q, and for its
+// ghosts (cells of earlier tasks the task reads) the values stored so far. It
+// leaves y0 = W q and the ghosts in the task's value table.
+//
+// Walk: pass by pass (a level, cut to the positions a warp holds at NB lanes
+// each), one lane per row of a cell: psi_row = y0_row - sum_slots G_row .
+// psi(up), the upwind values from the value table. What does not depend on
+// other cells (y0, the G row, the links) is read one pass ahead, so a pass's
+// critical path is the read of the upwind values, NB multiply-adds per slot
+// and the store: about 240 cycles alone and 370 among 16 warps per SM (FP32
+// triangles), against 520 for a lane per cell with all its rows. A task has
+// 2 to 6 cells per level, so rows and not cells fill the lanes.
+template <typename T, int NB, int F, int S, int KU, bool CACHED>
+__global__ void __launch_bounds__(64, SweepMinBlocks<T, NB, S, KU>()) SweepKernel(const DevGeom<T> g, const SweepDev s,
+                                                                                 const T *__restrict__ q,
+                                                                                 T *__restrict__ psi,
+                                                                                 const T *__restrict__ fac)
+{
+   extern __shared__ __align__(128) unsigned char smem_raw[];
+   const int lane = threadIdx.x & 31;
+   constexpr int EL = (int)sizeof(T);
+   constexpr int IP = 32 / NB;        // positions of one pass
+   constexpr int GC = S * NB * NB;    // coupling elements of a position
+   constexpr int GP = CACHED ? GC : LaneStride(GC, EL);
+   constexpr int SW = SchedWords(F);
+   constexpr size_t R = (size_t)NB * NB * (1 + S);
+   const SweepSlice L(s.P, S, F, NB, s.n_loc, s.n_ghost, EL, CACHED);
+   unsigned char *slice = smem_raw + (size_t)(threadIdx.x >> 5) * L.bytes;
+   uint64_t *bar = reinterpret_cast<uint64_t *>(slice + L.bar);
+   T *table = reinterpret_cast<T *>(slice + L.loc), *loc = table + NB;
+   uint16_t *pass = reinterpret_cast<uint16_t *>(slice + L.pass);
+   int32_t *gcell = reinterpret_cast<int32_t *>(slice + L.ghost);
+   const T *never = reinterpret_cast<const T *>(s.ctrl + kCtrlNever);
+   // A lane's position within a pass and its row (a spare lane: a position
+   // past every pass)
+   const int li = lane < IP * NB ? lane / NB : 1 << 20, lr = lane % NB;
+   // The factor store is read once per sweep: its lines go first from L2, so
+   // that they do not push out psi and the schedule other warps are reading
+   const uint64_t stream_once = EvictFirstPolicy();
+   if (lane < NB) table[lane] = T(0);
+   if (CACHED && lane == 0) {
+      MbarInit(bar, 1);
+      MbarInitFence();
+   }
+   __syncwarp();
+   uint32_t phase = 0;
+   for (;;) {
+      // A task is claimed only when the warp is free: a task claimed while
+      // the warp still walks (and waits in) another would sit idle behind it,
+      // and the tasks downstream of it would wait too (claiming even two
+      // levels before the walk ends measured slower)
+      const int64_t t = __shfl_sync(0xffffffffu, AtomicIncIf(lane == 0, &s.ctrl[kCtrlCounter]), 0);
+      if (t >= s.n_tasks) break;
+      const Task tk = LoadTask(s.task + t);
+      const int ncell = tk.ncell(), npass = tk.npass(), nghost = tk.nghost();
+      const int64_t off = tk.off;
+      const int a = tk.ordinate;
+      const int64_t base = (int64_t)tk.patch * s.P;
+      const bool hook = (t == s.unmet_task);
+      T *G = reinterpret_cast<T *>(slice + L.G);
+      const T *ft = fac + (size_t)off * R;
+      if constexpr (CACHED) {
+         // A bulk copy moves whole 16-byte units: from the unit the couplings
+         // start in (the store has a spare unit at its end)
+         const uintptr_t src = reinterpret_cast<uintptr_t>(ft + NB * NB * ncell);
+         const int lead = (int)(src & 15);
+         G += lead / EL;
+         const uint32_t bytes = (uint32_t)(lead + GC * ncell * EL + 15) & ~15u;
+         BulkLoadIf(lane == 0, slice + L.G, reinterpret_cast<const void *>(src - lead), bytes, bar, stream_once);
+      }
+      // No lane branches on its own below: a lane past the end repeats the last
+      // position or ghost (the same values to the same place)
+      const int32_t *gid = s.ghost + tk.ghost0;
+      const T *psi_a = psi + a * s.os_a;
+      const int glast = max(nghost - 1, 0);
+      const int32_t gh[2] = {gid[min(lane, glast)], gid[min(lane + 32, glast)]};
+      const uint16_t pass_word = s.pass[tk.pass0 + min(lane, npass - 1)];
+#pragma unroll 1
+      for (int i0 = 0; i0 < ncell; i0 += 32 * KU) {
+         using Rec = typename std::conditional<SW == 4, uint2, uint4>::type;
+         Rec rec[KU];
+         T W[KU][NB][NB], r[KU][NB], gx[2][NB];
+         int at[KU];
+#pragma unroll
+         for (int k = 0; k < KU; k++) {
+            const int i = at[k] = min(i0 + 32 * k + lane, ncell - 1);
+            rec[k] = __ldg(reinterpret_cast<const Rec *>(s.sched) + off + i);
+            if constexpr (CACHED)
+#pragma unroll
+               for (int e = 0; e < NB * NB; e++) W[k][e / NB][e % NB] = LoadHint(ft + (e * ncell + i), stream_once);
+         }
+         if (i0 == 0 && nghost > 0) {
+            // The ghosts' values where stored already, else the sentinel
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+               if (k == 1 && nghost <= 32) break;
+#pragma unroll
+               for (int j = 0; j < NB; j++) gx[k][j] = LoadRelaxed(psi_a + gh[k] * s.os_c + j * s.os_j);
+            }
+         }
+#pragma unroll
+         for (int k = 0; k < KU; k++) {
+            const int64_t c = base + (int)(rec[k].x & 0xffffu);
+            if (!s.aff_phi) {
+               const T *qc = q + c * s.qs_c + a * s.qs_a;
+#pragma unroll
+               for (int j = 0; j < NB; j++) r[k][j] = qc[j * s.qs_j];
+            } else {
+               const double ua = s.aff_u ? (double)static_cast<const T *>(s.aff_u)[a] : 1.0;
+               const double *ph = s.aff_phi + c * NB;
+               if (!s.aff_iso) {
+                  const double al = *s.aff_alpha;
+                  const T *qc = q + c * s.qs_c + a * s.qs_a;
+                  const double *rh = s.aff_rho + c * NB;
+#pragma unroll
+                  for (int j = 0; j < NB; j++) r[k][j] = (T)(al * (double)qc[j * s.qs_j] + ua * (ph[j] - al * rh[j]));
+               } else if (s.aff_inv_volume) {
+                  const double v = (double)g.volume[c];
+#pragma unroll
+                  for (int j = 0; j < NB; j++) r[k][j] = (T)(ua * ph[j] / v);
+               } else {
+#pragma unroll
+                  for (int j = 0; j < NB; j++) r[k][j] = (T)(ua * ph[j]);
+               }
+            }
+         }
+#pragma unroll
+         for (int k = 0; k < KU; k++) {
+            const int i = at[k];
+            if constexpr (!CACHED) {
+               if (i0 + 32 * k + lane >= ncell) continue;
+               const T om[3] = {g.omega[3 * a], g.omega[3 * a + 1], g.omega[3 * a + 2]};
+               T *Gi = G + i * GP;
+               const uint32_t mask = s.tmask[off + i];
+               CellFactors<T, NB, F>(g, base + (int)(rec[k].x & 0xffffu), om, mask, W[k], Gi, (size_t)NB,
+                                     (size_t)S * NB, 1);
+               ZeroSlots<T, NB>(Gi, __popc((mask | (mask >> 8)) & 0xffu), S);
+            }
+#pragma unroll
+            for (int ii = 0; ii < NB; ii++) {
+               T u = T(0);
+#pragma unroll
+               for (int j = 0; j < NB; j++) u += W[k][ii][j] * r[k][j];
+               loc[i * NB + ii] = u;
+            }
+            reinterpret_cast<Rec *>(slice + L.rec)[i] = rec[k];
+         }
+         if (i0 == 0 && nghost > 0) {
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+               if (k == 1 && nghost <= 32) break;
+               const int i = min(lane + 32 * k, glast);
+               gcell[i] = gh[k];
+#pragma unroll
+               for (int j = 0; j < NB; j++) loc[(ncell + i) * NB + j] = hook ? Sentinel<T>() : gx[k][j];
+            }
+         }
+      }
+      // Past the last pass the array repeats its end: two lookahead reads
+      if (lane < 2) pass[npass + lane] = (uint16_t)ncell;
+      pass[min(lane, npass - 1)] = pass_word;
+      for (int i0 = 32; i0 < npass; i0 += 32) {
+         const int i = min(i0 + lane, npass - 1);
+         pass[i] = s.pass[tk.pass0 + i];
+      }
+      for (int i0 = 64; i0 < nghost; i0 += 32) {
+         const int i = min(i0 + lane, glast);
+         const T *up = psi_a + gid[i] * s.os_c;
+         gcell[i] = gid[i];
+#pragma unroll
+         for (int j = 0; j < NB; j++) {
+            const T v = LoadRelaxed(up + j * s.os_j);
+            loc[(ncell + i) * NB + j] = hook ? Sentinel<T>() : v;
+         }
+      }
+      if constexpr (CACHED) {
+         // The couplings are in
+         if (!MbarWaitBounded(bar, phase, kCopyTries)) {
+            atomicOr(&s.ctrl[kCtrlError], 1u);
+            atomicAdd(&s.ctrl[kCtrlError + 1], 1u);
+            MbarWaitBounded(bar, phase, kCopyTries);
+            return;
+         }
+      }
+      phase ^= 1u;
+      __syncwarp();
+
+      // The walk. Every lane runs every pass (a branch that splits a warp cost
+      // 100 cycles a pass and more, as much as the pass itself); a lane
+      // without a row repeats position 0 and stores nothing
+      unsigned char *out = reinterpret_cast<unsigned char *>(psi + base * s.os_c + lr * s.os_j + a * s.os_a);
+      const int cell_bytes = (int)s.os_c * EL;
+      const T *Gr = G + lr * (S * NB);
+      const int ghost_from = (1 + ncell) * NB;
+      struct Own {  // what a row needs besides the upwind values
+         T y, g[S * NB];
+         uint16_t rec[SW];
+         int pos;
+         bool act;
+      };
+      auto fetch = [&](Own &o, int p0, int p1) {
+         o.act = p0 + li < p1;
+         o.pos = o.act ? p0 + li : 0;
+         memcpy(o.rec, slice + L.rec + o.pos * (SW * 2), SW * 2);
+         o.y = loc[o.pos * NB + lr];
+         LoadRow<T, S * NB, NB == 4>(Gr + o.pos * GP, o.g);
+      };
+      int p1 = pass[0], p2 = pass[1], l = 0;
+      auto step = [&](Own &cur, Own &nxt) {
+         T x[S][NB];
+#pragma unroll
+         for (int sl = 0; sl < S; sl++)
+            LoadRow<T, NB, NB == 4>(table + cur.rec[1 + sl], x[sl]);
+         // While those are on their way, the next pass's own data
+         fetch(nxt, p1, p2);
+         p1 = p2;
+         p2 = pass[l + 2];
+         // The row as if every ghost were there; then whether one may be
+         // missing, by the sentinel's upper word alone
+         auto row = [&]() {
+            T v = cur.y;
+#pragma unroll
+            for (int sl = 0; sl < S; sl++) {
+               T u = T(0);
+#pragma unroll
+               for (int j = 0; j < NB; j++) u += cur.g[sl * NB + j] * x[sl][j];
+               v -= u;
+            }
+            return v;
+         };
+         T yr = row();
+         uint32_t top = 0;
+#pragma unroll
+         for (int sl = 0; sl < S; sl++)
+#pragma unroll
+            for (int j = 0; j < NB; j++) top = max(top, TopWord(x[sl][j]));
+         if (__any_sync(0xffffffffu, cur.act && top == 0xffffffffu)) {
+            // Poll, one value per lane, a window of ghosts from the first
+            // missing one this pass reads: the ghosts are numbered in the order
+            // the passes read them, so the window holds what the next passes
+            // wait for too, and they find it in the value table (polling
+            // this pass's ghosts alone cost every later pass that reads a late
+            // one a round trip of its own). Bounded: on giving up the sticky
+            // error flag is set, the timeout counted, and this pass's missing
+            // values read as zero
+            for (uint32_t spins = 0;;) {
+               int first = nghost;
+#pragma unroll
+               for (int sl = 0; sl < S; sl++) {
+                  const int link = cur.rec[1 + sl];
+                  const bool need = cur.act && link >= ghost_from &&
+                                    IsSentinel(table[link + lr]);
+                  first = need ? min(first, (link - ghost_from) / NB) : first;
+               }
+               const bool mine_missing = first < nghost;
+               first = __reduce_min_sync(0xffffffffu, first);
+               if (first == nghost) break;
+               const int w = first + min(li, IP), i = min(w, glast), at = (ncell + i) * NB + lr;
+               T v = loc[at];
+               const bool ask = lane < IP * NB && w < nghost && IsSentinel(v);
+               // (test hook: this wait can never be met)
+               const T *src = hook ? never : psi_a + gcell[i] * s.os_c + lr * s.os_j;
+               LoadRelaxedIf(ask, src, v);
+               StoreSharedIf(ask, &loc[at], v);
+               __syncwarp();
+               // The error flag (another wait gave up) is read once per 1024
+               // spins, so that waiting lanes stay off its line
+               if (++spins > s.spin_limit ||
+                   ((spins & 1023u) == 0 && __any_sync(0xffffffffu, *(volatile uint32_t *)&s.ctrl[kCtrlError]))) {
+                  if (mine_missing) {
+                     atomicOr(&s.ctrl[kCtrlError], 1u);
+                     atomicAdd(&s.ctrl[kCtrlError + 1], 1u);
+                  }
+#pragma unroll
+                  for (int sl = 0; sl < S; sl++) {
+                     T *own = table + cur.rec[1 + sl] + lr;
+                     StoreSharedIf(cur.act && cur.rec[1 + sl] >= ghost_from && IsSentinel(*own), own, T(0));
+                  }
+                  __syncwarp();
+                  break;
+               }
+               if (spins > 64) __nanosleep(spins < 4096 ? 32 : 256);
+            }
+#pragma unroll
+            for (int sl = 0; sl < S; sl++) LoadRow<T, NB, NB == 4>(table + cur.rec[1 + sl], x[sl]);
+            yr = row();
+         }
+         StoreSharedIf(cur.act, &loc[cur.pos * NB + lr], yr);
+         StoreRelaxedIf(cur.act, reinterpret_cast<T *>(out + cur.rec[0] * cell_bytes), Publishable(yr));
+         __syncwarp();
+      };
+      Own own_a, own_b;
+      fetch(own_a, 0, p1);
+      while (true) {
+         step(own_a, own_b);
+         if (++l == npass) break;
+         step(own_b, own_a);
+         if (++l == npass) break;
+      }
+      __syncwarp();
+   }
+}
+
 // ~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~~
 
 static int ReserveFactors(ubolt_ctx *ctx, int64_t limit);
+
+// Couplings kept per cell: the kernels are built for 2 on triangles, 2 or 3
+// on quadrilaterals and tetrahedra, 3 or 5 on hexahedra
+static int SweepSlots(int F, int max_inflow)
+{
+   const int least = F == 6 ? 3 : 2;
+   return max_inflow <= least ? least : F - 1;
+}
 
 // The wave plan and both precisions' store layouts (host work and uploads;
 // no store is reserved here). Leaves wave_ok false where the mesh has an
@@ -625,37 +793,97 @@ int BuildSweepPlan(ubolt_ctx *ctx, int patch_size)
       return SetError(UBOLT_ERR_ARG, "a cell has %d upwind faces for one ordinate (at most %d)", h.max_inflow, ctx->F - 1);
    }
    plan->total_levels = (int64_t)h.lvl.size();
-   const int S = std::max(1, std::min(ctx->F - 1, (int)h.max_inflow));
-   plan->slots = S;
-   // The upwind link of every gathered face, in face order: the task's own
-   // cell (-2 - local) or a cell of an earlier task (its id)
-   std::vector<int32_t> tlink(h.tcell.size() * S, -1);
-   for (int64_t t = 0; t < h.n_tasks; t++) {
-      const int64_t base = (int64_t)(h.task_pa[t] / h.A) * h.P;
-      for (int64_t e = h.cell_ptr[t]; e < h.cell_ptr[t + 1]; e++) {
-         const int64_t c = base + h.tcell[e];
-         const uint32_t mask = h.tmask[e];
-         int slot = 0;
-         for (int f = 0; f < ctx->F; f++) {
-            const bool here = (mask >> f) & 1u, earlier = (mask >> (8 + f)) & 1u;
-            if (!(here || earlier)) continue;
-            const int32_t code = ctx->h_code[c * ctx->F + f];
-            tlink[e * S + slot++] = earlier ? code : (int32_t)(-2 - (code - base));
+   plan->slots = SweepSlots(ctx->F, h.max_inflow);
+   // Every entry's schedule record, with the upwind cells' places in the
+   // task's value table in face order; the cells of earlier tasks a task reads
+   // (its ghosts); and the passes, a level cut to the positions a warp walks
+   // at nb lanes each. Each thread takes a run of tasks and appends to lists
+   // of its own, joined in order
+   const int per_pass = 32 / ctx->nb, SW = SchedWords(ctx->F), nb = ctx->nb;
+   std::vector<uint16_t> sched(h.tcell.size() * SW, 0);
+   std::vector<Task> task(h.n_tasks);
+   const int n_parts = (int)std::min<int64_t>(std::max<int64_t>(1, h.n_tasks / 256), 256);
+   struct Part {
+      std::vector<uint16_t> pass;
+      std::vector<int32_t> ghost;
+      int n_loc = 0, n_ghost = 1;
+   };
+   std::vector<Part> part(n_parts);
+#pragma omp parallel for schedule(dynamic, 1)
+   for (int k = 0; k < n_parts; k++) {
+      Part &out = part[k];
+      std::vector<int32_t> pos_of(h.P, 0), mine;
+      for (int64_t t = h.n_tasks * k / n_parts; t < h.n_tasks * (k + 1) / n_parts; t++) {
+         const int64_t base = (int64_t)(h.task_pa[t] / h.A) * h.P, e0 = h.cell_ptr[t];
+         const int ncell = (int)(h.cell_ptr[t + 1] - e0);
+         mine.clear();
+         for (int i = 0; i < ncell; i++) pos_of[h.tcell[e0 + i]] = i;
+         for (int i = 0; i < ncell; i++) {
+            const int64_t c = base + h.tcell[e0 + i];
+            const uint32_t mask = h.tmask[e0 + i];
+            uint16_t *rec = &sched[(e0 + i) * SW];
+            rec[0] = h.tcell[e0 + i];
+            int slot = 0;
+            for (int f = 0; f < ctx->F; f++) {
+               const bool here = (mask >> f) & 1u, earlier = (mask >> (8 + f)) & 1u;
+               if (!(here || earlier)) continue;
+               const int32_t code = ctx->h_code[c * ctx->F + f];
+               int at = here ? pos_of[code - base] : 0;
+               if (earlier) {
+                  const auto it = std::find(mine.begin(), mine.end(), code);
+                  at = ncell + (int)(it - mine.begin());
+                  if (it == mine.end()) mine.push_back(code);
+               }
+               rec[1 + slot++] = (uint16_t)((1 + at) * nb);
+            }
          }
+         out.n_loc = std::max(out.n_loc, ncell + (int)mine.size() + 1);
+         out.n_ghost = std::max(out.n_ghost, (int)mine.size());
+         const size_t pass0 = out.pass.size();
+         int p0 = 0;
+         for (int32_t L = h.lvl_ptr[t]; L < h.lvl_ptr[t + 1]; L++) {
+            for (; p0 + per_pass < (int)h.lvl[L]; p0 += per_pass) out.pass.push_back((uint16_t)(p0 + per_pass));
+            p0 = h.lvl[L];
+            out.pass.push_back((uint16_t)p0);
+         }
+         Task &tk = task[t];
+         tk.counts = (uint32_t)ncell | (uint32_t)(out.pass.size() - pass0) << 10 | (uint32_t)mine.size() << 20;
+         tk.patch = h.task_pa[t] / h.A;
+         tk.ordinate = h.task_pa[t] % h.A;
+         tk.off = e0;
+         tk.ghost0 = (int64_t)out.ghost.size();
+         tk.pass0 = (int32_t)pass0;
+         out.ghost.insert(out.ghost.end(), mine.begin(), mine.end());
       }
    }
-   std::vector<uint16_t> tlev(h.tcell.size(), 0);
-   for (int64_t t = 0; t < h.n_tasks; t++) {
-      int64_t e = h.cell_ptr[t];
-      for (int32_t L = h.lvl_ptr[t]; L < h.lvl_ptr[t + 1]; L++)
-         for (; e < h.cell_ptr[t] + h.lvl[L]; e++) tlev[e] = (uint16_t)(L - h.lvl_ptr[t]);
+   std::vector<int64_t> pass_at(n_parts + 1, 0), ghost_at(n_parts + 1, 0);
+   for (int k = 0; k < n_parts; k++) {
+      pass_at[k + 1] = pass_at[k] + (int64_t)part[k].pass.size();
+      ghost_at[k + 1] = ghost_at[k] + (int64_t)part[k].ghost.size();
+      plan->n_loc = std::max(plan->n_loc, part[k].n_loc);
+      plan->n_ghost = std::max(plan->n_ghost, part[k].n_ghost);
+   }
+   if (pass_at[n_parts] >= INT32_MAX) {
+      delete plan;
+      return SetError(UBOLT_ERR_ARG, "too many sweep levels");
+   }
+   std::vector<uint16_t> pass(pass_at[n_parts]);
+   // A spare element, which a last task without ghosts reads (and does not use)
+   std::vector<int32_t> ghost(ghost_at[n_parts] + 1, 0);
+#pragma omp parallel for schedule(dynamic, 1)
+   for (int k = 0; k < n_parts; k++) {
+      std::copy(part[k].pass.begin(), part[k].pass.end(), pass.begin() + pass_at[k]);
+      std::copy(part[k].ghost.begin(), part[k].ghost.end(), ghost.begin() + ghost_at[k]);
+      for (int64_t t = h.n_tasks * k / n_parts; t < h.n_tasks * (k + 1) / n_parts; t++) {
+         task[t].pass0 += (int32_t)pass_at[k];
+         task[t].ghost0 += ghost_at[k];
+      }
    }
    int rc = 0;
-   if ((rc = UploadVec(ctx, h.task_pa, &plan->task_pa)) || (rc = UploadVec(ctx, h.dep_ptr, &plan->dep_ptr)) ||
-       (rc = UploadVec(ctx, h.deps, &plan->deps)) || (rc = UploadVec(ctx, h.cell_ptr, &plan->cell_ptr)) ||
-       (rc = UploadVec(ctx, h.tcell, &plan->tcell)) || (rc = UploadVec(ctx, h.tmask, &plan->tmask)) ||
-       (rc = UploadVec(ctx, h.lvl_ptr, &plan->lvl_ptr)) || (rc = UploadVec(ctx, h.lvl, &plan->lvl)) ||
-       (rc = UploadVec(ctx, tlink, &plan->tlink)) || (rc = UploadVec(ctx, tlev, &plan->tlev))) {
+   if ((rc = UploadVec(ctx, task, &plan->task)) || (rc = UploadVec(ctx, h.dep_ptr, &plan->dep_ptr)) ||
+       (rc = UploadVec(ctx, h.deps, &plan->deps)) || (rc = UploadVec(ctx, sched, &plan->sched)) ||
+       (rc = UploadVec(ctx, h.tmask, &plan->tmask)) || (rc = UploadVec(ctx, pass, &plan->pass)) ||
+       (rc = UploadVec(ctx, ghost, &plan->ghost))) {
       delete plan;
       return rc;
    }
@@ -682,14 +910,13 @@ static SweepDev DevPlan(const ubolt_sweep_plan *pl)
    s.P = pl->P;
    s.A = pl->A;
    s.n_tasks = pl->n_tasks;
-   s.task_pa = pl->task_pa;
-   s.cell_ptr = pl->cell_ptr;
-   s.tcell = pl->tcell;
+   s.task = pl->task;
+   s.sched = pl->sched;
    s.tmask = pl->tmask;
-   s.tlev = pl->tlev;
-   s.tlink = pl->tlink;
-   s.lvl_ptr = pl->lvl_ptr;
-   s.lvl = pl->lvl;
+   s.ghost = pl->ghost;
+   s.n_loc = pl->n_loc;
+   s.n_ghost = pl->n_ghost;
+   s.pass = pl->pass;
    s.ctrl = pl->ctrl;
    s.spin_limit = pl->spin_limit;
    s.unmet_task = -1;
@@ -701,20 +928,74 @@ static SweepDev DevPlan(const ubolt_sweep_plan *pl)
    return s;
 }
 
-// psi's layout for the task kernel
-static void SetLayout(SweepDev &s, const ubolt_ctx *ctx, bool ordinate_major)
+// The layouts of psi and of q for the task kernel
+static void SetLayout(SweepDev &s, const ubolt_ctx *ctx, bool psi_om, bool q_om)
 {
    const int64_t nb = ctx->nb, A = ctx->A;
-   if (ordinate_major) {
-      s.os_c = nb;
-      s.os_j = 1;
-      s.os_a = ctx->n_cells * nb;
+   s.os_c = psi_om ? nb : nb * A;
+   s.os_j = psi_om ? 1 : A;
+   s.os_a = psi_om ? ctx->n_cells * nb : 1;
+   s.qs_c = q_om ? nb : nb * A;
+   s.qs_j = q_om ? 1 : A;
+   s.qs_a = q_om ? ctx->n_cells * nb : 1;
+}
+
+// Between UBOLT's rows, x[node A + a], and ordinate-major, y[a n_nodes + node]:
+// a block moves 64 nodes of up to 64 ordinates through shared memory, so that
+// both its reads and its writes are runs of whole sectors. Bound by bandwidth.
+constexpr int kTransNodes = 64, kTransOrds = 64;
+template <typename T, bool TO_OM>
+__global__ void __launch_bounds__(256) TransposeKernel(const T *__restrict__ in, T *__restrict__ out, int A, int chunk,
+                                                       int64_t n_nodes)
+{
+   __shared__ T tile[kTransNodes][kTransOrds + 1];
+   const int64_t node0 = (int64_t)blockIdx.x * kTransNodes;
+   const int a0 = blockIdx.y * chunk, na = min(chunk, A - a0);
+   const int nn = (int)min((int64_t)kTransNodes, n_nodes - node0);
+   const int lane = threadIdx.x & 63, part = threadIdx.x >> 6;
+   // e / na for e < 4096 and na <= 64 (exact: e * na < 2^20)
+   const unsigned magic = ((1u << 20) + na - 1) / na;
+   if (TO_OM) {
+#pragma unroll 4
+      for (int e = threadIdx.x; e < nn * na; e += 256) {
+         const int n = (int)((e * magic) >> 20), a = e - n * na;
+         tile[n][a] = in[(node0 + n) * A + a0 + a];
+      }
+      __syncthreads();
+      if (lane < nn)
+#pragma unroll 4
+         for (int a = part; a < na; a += 4) out[(int64_t)(a0 + a) * n_nodes + node0 + lane] = tile[lane][a];
    } else {
-      s.os_c = nb * A;
-      s.os_j = A;
-      s.os_a = 1;
+      if (lane < nn)
+#pragma unroll 4
+         for (int a = part; a < na; a += 4) tile[lane][a] = in[(int64_t)(a0 + a) * n_nodes + node0 + lane];
+      __syncthreads();
+#pragma unroll 4
+      for (int e = threadIdx.x; e < nn * na; e += 256) {
+         const int n = (int)((e * magic) >> 20), a = e - n * na;
+         out[(node0 + n) * A + a0 + a] = tile[n][a];
+      }
    }
 }
+
+template <typename T>
+static void Transpose2(const ubolt_ctx *ctx, const T *in, T *out, bool to_om, cudaStream_t st)
+{
+   const int parts = (ctx->A + kTransOrds - 1) / kTransOrds, chunk = (ctx->A + parts - 1) / parts;
+   const dim3 grid((unsigned)((ctx->n_nodes + kTransNodes - 1) / kTransNodes), (unsigned)parts);
+   if (to_om) TransposeKernel<T, true><<<grid, 256, 0, st>>>(in, out, ctx->A, chunk, ctx->n_nodes);
+   else TransposeKernel<T, false><<<grid, 256, 0, st>>>(in, out, ctx->A, chunk, ctx->n_nodes);
+   CountLaunch();
+}
+
+// x in UBOLT's rows to ordinate-major y
+template <typename T>
+void ToOrdinateMajor(ubolt_ctx *ctx, const T *x, T *y, cudaStream_t st)
+{
+   Transpose2<T>(ctx, x, y, true, st);
+}
+template void ToOrdinateMajor<double>(ubolt_ctx *, const double *, double *, cudaStream_t);
+template void ToOrdinateMajor<float>(ubolt_ctx *, const float *, float *, cudaStream_t);
 
 // Bytes of the factor store for one precision
 static int64_t FactorBytes(const ubolt_ctx *ctx, const ubolt_sweep_plan *pl, size_t elem)
@@ -738,7 +1019,9 @@ static bool WavePreferred(const ubolt_ctx *ctx) { return ctx->n_cells * (int64_t
 static int ReserveFactors(ubolt_ctx *ctx, int64_t limit)
 {
    ubolt_sweep_plan *pl = ctx->sweep;
-   if (pl->fac[0] || pl->fac[1]) cudaDeviceSynchronize();
+   if (pl->fac[0] || pl->fac[1] || pl->scratch) cudaDeviceSynchronize();
+   if (pl->scratch) cudaFree(pl->scratch);
+   pl->scratch = nullptr;
    for (int which = 0; which < 2; which++) {
       if (pl->fac[which]) cudaFree(pl->fac[which]);
       pl->fac[which] = nullptr;
@@ -762,13 +1045,20 @@ static int ReserveFactors(ubolt_ctx *ctx, int64_t limit)
       const int64_t bytes = wave ? pl->wave_bytes[which] : FactorBytes(ctx, pl, which ? 4 : 8);
       if (bytes > left) continue;
       void *p = nullptr;
-      if (cudaMalloc(&p, (size_t)bytes) != cudaSuccess) {
+      if (cudaMalloc(&p, (size_t)bytes + 16) != cudaSuccess) {  // a copy of whole 16-byte units may end past the last factor
          cudaGetLastError();
          continue;
       }
       pl->fac[which] = p;
       pl->fac_wave[which] = wave;
       left -= bytes;
+   }
+   const int64_t vec = ctx->n_rows * (int64_t)sizeof(double);
+   if (vec <= left && !(pl->fac_wave[0] && pl->fac_wave[1])) {
+      if (cudaMalloc(&pl->scratch, (size_t)vec) != cudaSuccess) {
+         cudaGetLastError();
+         pl->scratch = nullptr;
+      }
    }
    return UBOLT_OK;
 }
@@ -792,7 +1082,9 @@ static T *EnsureFactors(ubolt_ctx *ctx, cudaStream_t st)
    cudaGetDevice(&dev);
    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
    const int64_t grid = std::min<int64_t>((pl->n_tasks + 3) / 4, (int64_t)n_sm * 16);
-   FactorKernel<T, NB, F><<<(int)grid, 128, 0, st>>>(ctx->geom<T>(), DevPlan(pl), static_cast<T *>(pl->fac[which]));
+   const int smem = 4 * 32 * LaneStride(pl->slots * NB * NB, (int)sizeof(T)) * (int)sizeof(T);
+   if (smem > 48 * 1024) cudaFuncSetAttribute(FactorKernel<T, NB, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+   FactorKernel<T, NB, F><<<(int)grid, 128, smem, st>>>(ctx->geom<T>(), DevPlan(pl), static_cast<T *>(pl->fac[which]));
    if (CheckLaunch("sweep factors")) return nullptr;
    pl->fac_epoch[which] = ctx->group_epoch;
    return static_cast<T *>(pl->fac[which]);
@@ -800,7 +1092,7 @@ static T *EnsureFactors(ubolt_ctx *ctx, cudaStream_t st)
 
 template <typename T, int NB, int F>
 static int LaunchSweep(ubolt_ctx *ctx, const T *q, T *psi, cudaStream_t st, const SweepDev *affine = nullptr,
-                       bool ordinate_major = false)
+                       bool ordinate_major = false, bool q_om = false)
 {
    ubolt_sweep_plan *pl = ctx->sweep;
    const int which = sizeof(T) == 8 ? 0 : 1;
@@ -827,25 +1119,50 @@ static int LaunchSweep(ubolt_ctx *ctx, const T *q, T *psi, cudaStream_t st, cons
       }
       return WaveSweep(ctx, w, q, psi, fac, (int)sizeof(T), affine ? &in : nullptr, pl->wave_threads, st);
    }
-   const int threads = 32 * pl->warps_per_block;
-   const size_t smem = (size_t)pl->warps_per_block * SweepSlice(pl->P, pl->slots, NB, (int)sizeof(T)).bytes;
-   auto kern = fac ? (pl->P <= 32 ? SweepKernel<T, NB, F, 1, true>
-                                  : pl->P <= 64 ? SweepKernel<T, NB, F, 2, true> : SweepKernel<T, NB, F, 8, true>)
-                   : (pl->P <= 32 ? SweepKernel<T, NB, F, 1, false>
-                                  : pl->P <= 64 ? SweepKernel<T, NB, F, 2, false> : SweepKernel<T, NB, F, 8, false>);
-   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-   int per_sm = 0, n_sm = 0, dev = 0;
+   // Two warps per block; one where the patch's couplings leave no room for two
+   const size_t slice = (size_t)SweepSlice(pl->P, pl->slots, F, NB, pl->n_loc, pl->n_ghost, (int)sizeof(T), fac != nullptr).bytes;
+   constexpr int S0 = F == 6 ? 3 : 2;
+   // Two positions per lane in a prologue where the tasks hold more than a
+   // warp's worth, one where they are small (jittered tetrahedra: 8 cells of 24)
+   const bool wide = ctx->n_cells * (int64_t)ctx->A > 24 * pl->n_tasks;
+   auto kern = pl->slots == S0 ? (fac ? (wide ? SweepKernel<T, NB, F, S0, 2, true> : SweepKernel<T, NB, F, S0, 1, true>)
+                                      : (wide ? SweepKernel<T, NB, F, S0, 2, false> : SweepKernel<T, NB, F, S0, 1, false>))
+                               : (fac ? (wide ? SweepKernel<T, NB, F, F - 1, 2, true> : SweepKernel<T, NB, F, F - 1, 1, true>)
+                                      : (wide ? SweepKernel<T, NB, F, F - 1, 2, false> : SweepKernel<T, NB, F, F - 1, 1, false>));
+   int per_sm = 0, n_sm = 0, dev = 0, smem_max = 48 * 1024;
    cudaGetDevice(&dev);
    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+   cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+   const int warps = 2 * slice <= (size_t)smem_max ? 2 : 1, threads = 32 * warps;
+   const size_t smem = warps * slice;
+   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-   // At most 32 warps per SM: beyond the throughput the wavefront can use,
-   // more resident warps only take tasks early and wait
-   per_sm = std::min(per_sm, kSweepBlocksPerSm);
-   const int64_t want = (pl->n_tasks + pl->warps_per_block - 1) / pl->warps_per_block;
+   // At most 32 warps per SM (small DG0 tasks): beyond the throughput the
+   // wavefront can use, more resident warps only take tasks early and wait
+   per_sm = std::min(per_sm, kSweepWarpsPerSm / warps);
+   const int64_t want = (pl->n_tasks + warps - 1) / warps;
    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)std::max(per_sm, 1) * n_sm, want));
    pl->grid = grid;
    SweepDev s = DevPlan(pl);
-   SetLayout(s, ctx, ordinate_major);
+   // Row vectors in and out: in UBOLT's rows a task's values of one ordinate
+   // lie A apart, each its own sector in and out. Where there are several
+   // rows per cell and more than a few MB, the sweep itself runs
+   // ordinate-major, psi holding q's ordinate-major copy meanwhile and the
+   // scratch vector the result: two passes at memory bandwidth against the
+   // scattered words. Per sweep, FP64 / FP32, direct and this way: 256^2
+   // triangles 916 / 586 -> 702 / 564 us, 40^3 hexahedra 1094 / 900 -> 775 /
+   // 481, 20^3 cubes of tetrahedra 1278 / 890 -> 1054 / 576; DG0 quadrilaterals
+   // 244 -> 247 and a 1.1 M-row FP32 vector 151 -> 154, which stay direct
+   T *dst = psi;
+   const bool via = !ordinate_major && !q_om && pl->scratch && NB > 1 && ctx->n_rows * sizeof(T) >= kViaBytes;
+   if (via) {
+      if (!affine || !affine->aff_iso) {
+         Transpose2<T>(ctx, q, psi, true, st);
+         q = psi;
+      }
+      dst = static_cast<T *>(pl->scratch);
+   }
+   SetLayout(s, ctx, ordinate_major || via, q_om || via);
    if (affine) {
       s.aff_alpha = affine->aff_alpha;
       s.aff_phi = affine->aff_phi;
@@ -858,9 +1175,12 @@ static int LaunchSweep(ubolt_ctx *ctx, const T *q, T *psi, cudaStream_t st, cons
    pl->unmet_task = -1;
    cudaMemsetAsync(pl->ctrl + kCtrlCounter, 0, sizeof(uint32_t), st);  // task counter; the error flag stays sticky
    // Every psi value starts as the sentinel: "not yet stored by its task"
-   cudaMemsetAsync(psi, 0xff, (size_t)ctx->n_cells * NB * ctx->A * sizeof(T), st);
-   kern<<<grid, threads, smem, st>>>(ctx->geom<T>(), s, q, psi, fac);
-   return CheckLaunch("sweep");
+   cudaMemsetAsync(dst, 0xff, (size_t)ctx->n_cells * NB * ctx->A * sizeof(T), st);
+   kern<<<grid, threads, smem, st>>>(ctx->geom<T>(), s, q, dst, fac);
+   const int rc = CheckLaunch("sweep");
+   if (rc || !via) return rc;
+   Transpose2<T>(ctx, dst, psi, false, st);
+   return CudaCheck(cudaGetLastError(), "sweep");
 }
 
 template <typename T>

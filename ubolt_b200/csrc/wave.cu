@@ -34,51 +34,6 @@ namespace ubolt {
 
 namespace {
 
-__device__ __forceinline__ uint32_t SmemAddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void MbarInit(uint64_t *bar, uint32_t count)
-{
-   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(SmemAddr(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void MbarInitFence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-
-__device__ __forceinline__ void MbarExpectTx(uint64_t *bar, uint32_t bytes)
-{
-   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(SmemAddr(bar)), "r"(bytes) : "memory");
-}
-
-// One contiguous global -> shared copy completing on `bar` (both addresses
-// 16-byte aligned, bytes a multiple of 16)
-__device__ __forceinline__ void BulkLoad(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
-{
-   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                    SmemAddr(dst)),
-                "l"(src), "r"(bytes), "r"(SmemAddr(bar))
-                : "memory");
-}
-
-__device__ __forceinline__ bool MbarTryWait(uint64_t *bar, uint32_t parity)
-{
-   uint32_t ok;
-   asm volatile(
-       "{\n\t.reg .pred p;\n\t"
-       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-       "selp.u32 %0, 1, 0, p;\n\t}"
-       : "=r"(ok)
-       : "r"(SmemAddr(bar)), "r"(parity)
-       : "memory");
-   return ok != 0;
-}
-
-// At most limit + 1 polls of the phase
-__device__ __forceinline__ bool MbarWaitBounded(uint64_t *bar, uint32_t parity, uint32_t limit)
-{
-   for (uint32_t k = 0; k <= limit; k++)
-      if (MbarTryWait(bar, parity)) return true;
-   return false;
-}
-
 // One level's factor chunk: W, then the S couplings, element-major
 template <typename T>
 __host__ __device__ __forceinline__ uint32_t ChunkBytes(int width, int R)
@@ -104,7 +59,8 @@ __global__ void __launch_bounds__(128) WaveFactorKernel(const DevGeom<T> g, cons
          const int4 m = w.meta[(int64_t)a * w.n_cells + p0 + i];
          const uint32_t mask = ((uint32_t)m.y >> 16) & 0xffu;
          T W[NB][NB];
-         CellFactors<T, NB, F>(g, m.x, om, mask, W, ck + (size_t)NB * NB * n + i, (size_t)NB * NB * n, (size_t)n);
+         CellFactors<T, NB, F>(g, m.x, om, mask, W, ck + (size_t)NB * NB * n + i, (size_t)NB * NB * n,
+                               (size_t)NB * n, (size_t)n);
 #pragma unroll
          for (int ii = 0; ii < NB; ii++)
 #pragma unroll
