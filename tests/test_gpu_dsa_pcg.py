@@ -1,0 +1,62 @@
+"""The DSA's inner solve in one launch, where its layout changes: a few cells,
+one per thread with the matrix in shared memory, one per thread without, and
+more cells than threads. Against the same iteration in NumPy on the assembled
+matrix (whose entries tests/test_dsa.py checks against the oracle)."""
+import numpy as np
+import pytest
+import torch
+
+from ubolt_b200 import problem as P
+from ubolt_b200 import transport as T
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "one_block": (lambda r: P.box_tris(5, 3, jitter=0.2, rng=r), 1),
+    "blocks_and_a_rest": (lambda r: P.box_quads(45, 31, jitter=0.2, rng=r), 1),
+    "dg0": (lambda r: P.box_hexes(12, 11, 7), 0),
+    "tets_kept": (lambda r: P.box_tets(12, 12, 11, jitter=0.2, rng=r), 1),
+    "hexes_past_shared_memory": (lambda r: P.box_hexes(35, 34, 34), 1),
+    "more_cells_than_threads": (lambda r: P.box_tris(220, 190, jitter=0.2, rng=r), 1),
+}
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_inner_solve_matches_numpy(case):
+    make, order = CASES[case]
+    rng = np.random.default_rng(3)
+    m = make(rng)
+    g, q = P.build_geometry(m, order), P.lqn(m.dim, 2)
+    st = rng.uniform(0.5, 3.0, g.n_cells)
+    ss = st * rng.uniform(0.3, 0.9, g.n_cells)
+    ctx = T.Context(g, q)
+    keep = (torch.tensor(st, device="cuda"), torch.tensor(ss, device="cuda"))
+    ctx.set_group(*keep)
+    its = 6
+    dsa = T.DSAPrecon(ctx, inner_iterations=its)
+    dsa.set_group()
+    D, nb, A = dsa.matrix(), g.n_basis, q.n_angles
+    x = rng.standard_normal(ctx.n_rows)
+    rhs = np.repeat(g.volume, nb) * (x.reshape(-1, A) @ q.w)
+    rows = np.arange(g.n_cells * nb).reshape(-1, nb)
+    blocks = np.stack([np.asarray(D[rows[:, i], rows[:, j]]).ravel() for i in range(nb) for j in range(nb)],
+                      axis=1).reshape(-1, nb, nb)
+    jac = np.linalg.inv(blocks)
+    apply_j = lambda v: np.einsum("cij,cj->ci", jac, v.reshape(-1, nb)).ravel()
+    u, r = np.zeros_like(rhs), rhs.copy()
+    z = apply_j(r)
+    p, rho = z.copy(), r @ z
+    for _ in range(its):
+        s = D @ p
+        alpha = rho / (p @ s)
+        u, r = u + alpha * p, r - alpha * s
+        z = apply_j(r)
+        new = r @ z
+        p, rho = z + new / rho * p, new
+    ref = np.repeat(u / q.sum_weights, A)
+    y = dsa.apply(torch.tensor(x, device="cuda")).cpu().numpy()
+    # Six iterations amplify rounding by far less than 1e5
+    assert np.linalg.norm(y - ref) <= 1e-11 * np.linalg.norm(ref)
+    v = dsa.spmv(torch.tensor(rhs, device="cuda")).cpu().numpy()
+    assert np.linalg.norm(v - D @ rhs) <= 1e-13 * np.linalg.norm(D @ rhs)
+    ctx.close()

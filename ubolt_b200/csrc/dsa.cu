@@ -20,11 +20,12 @@
 // As in the reference the matrix is refilled on the host per group (a host
 // loop) and uploaded; here into a block-ELL layout - per cell its F neighbour
 // blocks (slot order, zero where a face has no neighbour) then its own block,
-// nb x nb each - so the SpMV is one gather per face, coalesced over nodes.
+// nb x nb each - stored element by element over the cells, so that a thread
+// per cell reads the matrix coalesced.
 // The inner solve replaces the reference's one GAMG V-cycle (PCGAMG,
 // dsak.kokkos.cxx:197-212) with a fixed number of block-Jacobi PCG
-// iterations run entirely on the device (scalars stay in device memory, no
-// host round trip), in FP64 whatever the outer precision.
+// iterations run entirely on the device in one cooperative launch (no host round
+// trip), in FP64 whatever the outer precision.
 //
 // On a CG-SUPG context the operator is DSACG's (src/dsa_cgk.kokkos.cxx): one
 // unknown per vertex, the weak form
@@ -70,112 +71,99 @@ struct ubolt_dsa {
    int64_t *d_rp = nullptr;
    int32_t *d_col = nullptr;
    // Device
-   double *val = nullptr, *jinv = nullptr;          // [nc][F+1][nb][nb], [nc][nb][nb] (CG: [nnz], [n_nodes])
+   double *val = nullptr, *jinv = nullptr;          // [F+1][nb][nb][nc], [nb][nb][nc] (CG: [nnz], [n_nodes])
    double *rhs = nullptr, *u = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr;
-   // [0] rho, [1] rho_new, [2] pq, [3] the grid sums' block counter (an
-   // unsigned int in a double's slot), then one partial per block
-   double *scal = nullptr;
+   double *slots = nullptr;  // the grid sums' counter (in two words' place), then two slots per block
 };
 
 namespace ubolt {
 
-constexpr int kDsaThreads = 256;
+// The PCG's blocks: one of 512 threads per SM (at two of 384 the kernel
+// spilled, and a spill is a trip to L2 here, as every grid sum empties L1), the
+// tries of a bounded wait, and the shared memory a block may hold of the matrix
+constexpr int kPcgThreads = 512, kPcgBlocksPerSm = 1;
+constexpr uint32_t kPcgTries = 1u << 24;
+constexpr int64_t kPcgKeepBytes = 220 * 1024;
+// A cell's matrix in shared memory, an odd number of values apart (no bank conflicts)
+__host__ __device__ constexpr int KeptStride(int F, int NB) { return (F + 1) * NB * NB | 1; }
 
-// Scalar slots ahead of the per-block partials
-constexpr int kDsaScalars = 4;
-
-// Deterministic sum of d over the grid into *out: each block's total goes to
-// part[blockIdx.x]; the last block to finish (an integer counter) adds the
-// totals in a fixed order - per-lane strided sums, then a shuffle tree, the
-// same every run - writes *out and resets the counter. No block waits on
-// another. Every thread of the block must call it.
-__device__ __forceinline__ void GridSum(double d, double *part, unsigned *count, double *out)
+// A cell's neighbours. A face without one has zero blocks: it reads the cell
+// itself, so that no lane branches on its own
+template <int F>
+__device__ __forceinline__ void CellNeighbours(int64_t c, const int32_t *__restrict__ code, int32_t (&nbr)[F])
 {
-   __shared__ double red[kDsaThreads / 32];
-   __shared__ bool last;
-   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
-   for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-   if (lane == 0) red[warp] = d;
-   __syncthreads();
-   if (threadIdx.x == 0) {
-      double s = 0.0;
-      for (int w = 0; w < nw; w++) s += red[w];
-      part[blockIdx.x] = s;
-      __threadfence();
-      last = atomicAdd(count, 1u) == gridDim.x - 1;
-   }
-   __syncthreads();
-   if (!last) return;
-   __threadfence();
-   double s = 0.0;
-   for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s += __ldcg(&part[b]);
-#pragma unroll
-   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-   __syncthreads();
-   if (lane == 0) red[warp] = s;
-   __syncthreads();
-   if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < nw; w++) t += red[w];
-      *out = t;
-      *count = 0;
+   for (int f = 0; f < F; f++) {
+      const int32_t n = code[c * F + f];
+      nbr[f] = n < 0 ? (int32_t)c : n;
    }
 }
 
-__device__ __forceinline__ unsigned *GridCount(double *scal) { return reinterpret_cast<unsigned *>(scal + 3); }
-
-// v = D u over the block-ELL rows, one thread per node
-__global__ void DsaSpmvKernel(int64_t n_nodes, int nb, int F, const int32_t *__restrict__ code,
-                              const double *__restrict__ val, const double *__restrict__ u, double *__restrict__ v,
-                              const double *__restrict__ dotw, double *scal)
+// sum_{f, j} D(i; f, j) x(f, j) over a cell's neighbours and itself for its NB
+// rows: x(cell, j) given by `at`, element k of the cell's matrix by `val`
+template <int NB, int F, typename Val, typename At>
+__device__ __forceinline__ void CellRows(const int32_t (&nbr)[F], Val val, const double (&own)[NB], At at, double (&s)[NB])
 {
-   const int64_t node = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-   double d = 0.0;
-   if (node < n_nodes) {
-      const int64_t c = node / nb;
-      const int i = (int)(node - c * nb);
-      const double *blk = val + (c * (F + 1)) * nb * nb;
-      double s = 0.0;
-      for (int f = 0; f < F; f++) {
-         const int32_t n = code[c * F + f];
-         if (n < 0) continue;
-         for (int j = 0; j < nb; j++) s += blk[(f * nb + i) * nb + j] * u[(int64_t)n * nb + j];
-      }
-      for (int j = 0; j < nb; j++) s += blk[(F * nb + i) * nb + j] * u[c * nb + j];
-      v[node] = s;
-      if (dotw) d = dotw[node] * s;
+#pragma unroll
+   for (int i = 0; i < NB; i++) s[i] = 0.0;
+#pragma unroll
+   for (int f = 0; f < F; f++) {
+      double x[NB];
+#pragma unroll
+      for (int j = 0; j < NB; j++) x[j] = at(nbr[f], j);
+#pragma unroll
+      for (int i = 0; i < NB; i++)
+#pragma unroll
+         for (int j = 0; j < NB; j++) s[i] += val((f * NB + i) * NB + j) * x[j];
    }
-   // scal[2] = (dotw, v), when asked
-   if (scal) GridSum(d, scal + kDsaScalars, GridCount(scal), &scal[2]);
+#pragma unroll
+   for (int i = 0; i < NB; i++)
+#pragma unroll
+      for (int j = 0; j < NB; j++) s[i] += val((F * NB + i) * NB + j) * own[j];
+}
+
+// v = D u over the block-ELL rows, one thread per cell
+template <int NB, int F>
+__global__ void __launch_bounds__(128) DsaSpmvKernel(int64_t nc, const int32_t *__restrict__ code,
+                                                     const double *__restrict__ val, const double *__restrict__ u,
+                                                     double *__restrict__ v)
+{
+   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+   if (c >= nc) return;
+   double own[NB], s[NB];
+#pragma unroll
+   for (int j = 0; j < NB; j++) own[j] = u[c * NB + j];
+   int32_t nbr[F];
+   CellNeighbours<F>(c, code, nbr);
+   CellRows<NB, F>(nbr, [&](int k) { return __ldg(val + (int64_t)k * nc + c); }, own,
+                   [&](int32_t n, int j) { return u[(int64_t)n * NB + j]; }, s);
+#pragma unroll
+   for (int i = 0; i < NB; i++) v[c * NB + i] = s[i];
 }
 
 // v = D u over CSR rows (the CG-SUPG vertices), one thread per row
 __global__ void DsaCsrSpmvKernel(int64_t n_nodes, const int64_t *__restrict__ rp, const int32_t *__restrict__ col,
-                                 const double *__restrict__ val, const double *__restrict__ u, double *__restrict__ v,
-                                 const double *__restrict__ dotw, double *scal)
+                                 const double *__restrict__ val, const double *__restrict__ u, double *__restrict__ v)
 {
    const int64_t node = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-   double d = 0.0;
-   if (node < n_nodes) {
-      double s = 0.0;
-      for (int64_t k = rp[node]; k < rp[node + 1]; k++) s += val[k] * u[col[k]];
-      v[node] = s;
-      if (dotw) d = dotw[node] * s;
-   }
-   if (scal) GridSum(d, scal + kDsaScalars, GridCount(scal), &scal[2]);
+   if (node >= n_nodes) return;
+   double s = 0.0;
+   for (int64_t k = rp[node]; k < rp[node + 1]; k++) s += val[k] * u[col[k]];
+   v[node] = s;
 }
 
-// v = D u in whichever storage the context's DSA has; with scal, also (dotw, v) into scal[2]
-static void DsaSpmvLaunch(const ubolt_ctx *ctx, const ubolt_dsa *ds, const double *u, double *v, const double *dotw,
-                          double *scal, cudaStream_t s)
+// v = D u in whichever storage the context's DSA has
+static int DsaSpmvLaunch(const ubolt_ctx *ctx, const ubolt_dsa *ds, const double *u, double *v, cudaStream_t s)
 {
-   const int64_t grid = (ds->n_nodes + kDsaThreads - 1) / kDsaThreads;
-   if (ds->cg)
-      DsaCsrSpmvKernel<<<grid, kDsaThreads, 0, s>>>(ds->n_nodes, ds->d_rp, ds->d_col, ds->val, u, v, dotw, scal);
-   else
-      DsaSpmvKernel<<<grid, kDsaThreads, 0, s>>>(ds->n_nodes, ds->nb, ds->F, ctx->g64.code, ds->val, u, v, dotw,
-                                                 scal);
+   if (ds->cg) {
+      DsaCsrSpmvKernel<<<(ds->n_nodes + 127) / 128, 128, 0, s>>>(ds->n_nodes, ds->d_rp, ds->d_col, ds->val, u, v);
+      return CheckLaunch("dsa_spmv");
+   }
+   UBOLT_DISPATCH(ds->nb, ds->F, {
+      DsaSpmvKernel<NB_, F_><<<(ds->nc + 127) / 128, 128, 0, s>>>(ds->nc, ctx->g64.code, ds->val, u, v);
+      return CheckLaunch("dsa_spmv");
+   });
+   return SetError(UBOLT_ERR_STATE, "no DSA kernel for this shape");
 }
 
 // rhs(node) = V_c sum_a w_a (x(node, a) - ax(node, a)); ax may be NULL. A
@@ -224,70 +212,250 @@ __global__ void __launch_bounds__(256) DsaProlongKernel(int64_t n_nodes, int nb,
 
 // ~~~ Block-Jacobi PCG on the device, a fixed number of iterations from u = 0
 
-// r = rhs, u = 0, z = J r, p = z, scal[0] = (r, z)
-__global__ void CgStartKernel(int64_t n_nodes, int nb, const double *__restrict__ jinv, const double *__restrict__ rhs,
-                              double *__restrict__ u, double *__restrict__ r, double *__restrict__ z,
-                              double *__restrict__ p, double *scal)
+struct DsaPcgArgs {
+   int64_t n;  // cells, or vertices (CSR)
+   int its;
+   const int32_t *code;
+   const int64_t *rp;
+   const int32_t *col;
+   const double *val, *jinv;
+   double *rhs;  // the right-hand side; from the first iteration on, the odd directions
+   double *u, *r, *z, *p, *q;
+   unsigned *count;  // blocks arrived, zero at launch
+   double *slots;    // [2][blocks], see GridSum
+};
+
+// The sum of d over the grid, the same bits in every thread, and with it a grid
+// barrier: each block leaves its share in slots[step parity][block], arrives on
+// the counter and waits for all blocks; then the shares are added in a fixed
+// order. Bounded; false (in every thread of the block): gave up. About 1.3 us
+// with 296 blocks and one thread of each polling the counter; every block
+// polling every other's slot instead took 6 us.
+__device__ __forceinline__ bool GridSum(double d, const DsaPcgArgs &a, unsigned step, double *sum)
 {
-   const int64_t node = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-   double d = 0.0;
-   if (node < n_nodes) {
-      const int64_t c = node / nb;
-      const int i = (int)(node - c * nb);
-      double zz = 0.0;
-      for (int j = 0; j < nb; j++) zz += jinv[(c * nb + i) * nb + j] * rhs[c * nb + j];
-      r[node] = rhs[node];
-      u[node] = 0.0;
-      z[node] = zz;
-      p[node] = zz;
-      d = rhs[node] * zz;
+   constexpr int kWarps = kPcgThreads / 32;
+   __shared__ double red[kWarps], total;
+   __shared__ int ok;
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = gridDim.x;
+   double *row = a.slots + (step & 1) * G;
+#pragma unroll
+   for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+   if (lane == 0) red[warp] = d;
+   __syncthreads();
+   if (warp == 0) {
+      if (lane == 0) {
+         double s = 0.0;
+#pragma unroll
+         for (int w = 0; w < kWarps; w++) s += red[w];
+         row[blockIdx.x] = s;
+         // The block's writes of this phase before its arrival (its threads met above)
+         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.count) : "memory");
+         const unsigned target = (step + 1) * (unsigned)G;
+         unsigned v;
+         uint32_t tries = 0;
+         do {
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.count) : "memory");
+         } while (v < target && ++tries < kPcgTries);
+         ok = v >= target;
+         __threadfence();
+      }
+      __syncwarp();
+      double t = 0.0;
+#pragma unroll 10
+      for (int b = lane; b < G; b += 32) t += __ldcg(row + b);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) total = t;
    }
-   GridSum(d, scal + kDsaScalars, GridCount(scal), &scal[0]);
+   __syncthreads();
+   *sum = total;
+   return ok;
 }
 
-// alpha = rho / pq; u += alpha p; r -= alpha q
-__global__ void CgUpdateKernel(int64_t n_nodes, const double *__restrict__ p, const double *__restrict__ q,
-                               double *__restrict__ u, double *__restrict__ r, const double *scal)
+// The whole inner solve in one cooperative launch: a block owns a run of
+// cells, a thread one cell at a time with all its rows, and an iteration is two
+// phases with a grid sum after each:
+//    p = z + beta p, q = D p, (p, q);   u += alpha p, r -= alpha q, z = J r, (r, z).
+// A neighbour's direction is formed from its z and its last p where it is
+// read (p alternates between two buffers), which saves a third barrier. OWN:
+// every thread has at most one cell, whose vectors stay in its registers, and
+// KEEP: its matrix rows stay in shared memory (a grid sum's fence empties L1).
+// Bound by the grid sums (about 2 us each with the sum) and one L2 round trip
+// per phase. Per apply (30 iterations, S8), the launch-by-launch form (five
+// kernels an iteration) and this one: 192^2 triangles 898 -> 368 us, 256^2 (more
+// cells than threads) 1266 -> 731, 32^3 hexahedra 905 -> 426, 16^3 cubes of
+// tetrahedra 832 -> 385, 24^2 triangles 667 -> 199.
+template <int NB, int F, bool CSR, bool OWN, bool KEEP>
+__global__ void __launch_bounds__(kPcgThreads, kPcgBlocksPerSm) DsaPcgKernel(const DsaPcgArgs a)
 {
-   const int64_t node = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-   if (node >= n_nodes) return;
-   const double pq = scal[2];
-   const double alpha = pq != 0.0 ? scal[0] / pq : 0.0;
-   u[node] += alpha * p[node];
-   r[node] -= alpha * q[node];
-}
-
-// z = J r; scal[1] = (r, z)
-__global__ void CgPrecondKernel(int64_t n_nodes, int nb, const double *__restrict__ jinv, const double *__restrict__ r,
-                                double *__restrict__ z, double *scal)
-{
-   const int64_t node = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-   double d = 0.0;
-   if (node < n_nodes) {
-      const int64_t c = node / nb;
-      const int i = (int)(node - c * nb);
-      double zz = 0.0;
-      for (int j = 0; j < nb; j++) zz += jinv[(c * nb + i) * nb + j] * r[c * nb + j];
-      z[node] = zz;
-      d = r[node] * zz;
+   extern __shared__ double kept[];  // KEEP: [cells of a block][KeptStride], a thread's run at fixed offsets
+   double *mine = kept + threadIdx.x * KeptStride(F, NB);
+   const int64_t per = (a.n + gridDim.x - 1) / gridDim.x;
+   const int64_t c0 = blockIdx.x * per, c1 = min(a.n, c0 + per);
+   unsigned step = 0;
+   // OWN, up to three rows: the thread's Jacobi block in registers
+   constexpr bool kJac = OWN && NB <= 3;
+   double jac[kJac ? NB * NB : 1];
+   int32_t nbr[F];
+   if (OWN && c0 + threadIdx.x < c1) {
+      const int64_t c = c0 + threadIdx.x;
+      if constexpr (kJac)
+#pragma unroll
+         for (int k = 0; k < NB * NB; k++) jac[k] = a.jinv[(int64_t)k * a.n + c];
+      if constexpr (!CSR) CellNeighbours<F>(c, a.code, nbr);
+      if constexpr (KEEP)
+#pragma unroll 8
+         for (int k = 0; k < (F + 1) * NB * NB; k++) mine[k] = a.val[(int64_t)k * a.n + c];
    }
-   GridSum(d, scal + kDsaScalars, GridCount(scal), &scal[1]);
+   auto precondition = [&](int64_t c, const double (&r)[NB], double (&z)[NB]) {
+      double d = 0.0;
+#pragma unroll
+      for (int i = 0; i < NB; i++) {
+         double s = 0.0;
+#pragma unroll
+         for (int j = 0; j < NB; j++) s += (kJac ? jac[kJac ? i * NB + j : 0] : __ldg(a.jinv + (int64_t)(i * NB + j) * a.n + c)) * r[j];
+         z[i] = s;
+         d += r[i] * s;
+      }
+      return d;
+   };
+   double u[NB], r[NB], z[NB], p[NB], q[NB], d = 0.0, rho = 0.0, beta = 0.0;
+   for (int64_t c = c0 + threadIdx.x; c < c1; c += kPcgThreads) {
+#pragma unroll
+      for (int i = 0; i < NB; i++) r[i] = a.rhs[c * NB + i];
+      d += precondition(c, r, z);
+#pragma unroll
+      for (int i = 0; i < NB; i++) {
+         u[i] = 0.0;
+         a.z[c * NB + i] = z[i];
+         if (!OWN) {
+            a.r[c * NB + i] = r[i];
+            a.u[c * NB + i] = 0.0;
+         }
+      }
+   }
+   bool ok = GridSum(d, a, step++, &rho);
+   for (int it = 0; it < a.its && ok; it++) {
+      double *p_now = it & 1 ? a.rhs : a.p;
+      const double *p_old = it & 1 ? a.p : a.rhs;
+      // Written by other blocks in an earlier phase: read past L1
+      auto direction = [&](int64_t k) {
+         const double zk = __ldcg(a.z + k);
+         return it ? zk + beta * __ldcg(p_old + k) : zk;
+      };
+      d = 0.0;
+      for (int64_t c = c0 + threadIdx.x; c < c1; c += kPcgThreads) {
+#pragma unroll
+         for (int j = 0; j < NB; j++) {
+            if constexpr (OWN) p[j] = it ? z[j] + beta * p[j] : z[j];
+            else p[j] = direction(c * NB + j);
+         }
+         if constexpr (CSR) {
+            q[0] = 0.0;
+            for (int64_t k = a.rp[c]; k < a.rp[c + 1]; k++) q[0] += __ldg(a.val + k) * direction(a.col[k]);
+         } else {
+            if constexpr (!OWN) CellNeighbours<F>(c, a.code, nbr);
+            auto at = [&](int32_t n, int j) { return direction((int64_t)n * NB + j); };
+            if constexpr (KEEP) CellRows<NB, F>(nbr, [&](int k) { return mine[k]; }, p, at, q);
+            else CellRows<NB, F>(nbr, [&](int k) { return __ldg(a.val + (int64_t)k * a.n + c); }, p, at, q);
+         }
+#pragma unroll
+         for (int i = 0; i < NB; i++) {
+            p_now[c * NB + i] = p[i];
+            if (!OWN) a.q[c * NB + i] = q[i];
+            d += p[i] * q[i];
+         }
+      }
+      double pq = 0.0;
+      if (!(ok = GridSum(d, a, step++, &pq))) break;
+      const double alpha = pq != 0.0 ? rho / pq : 0.0;
+      d = 0.0;
+      for (int64_t c = c0 + threadIdx.x; c < c1; c += kPcgThreads) {
+#pragma unroll
+         for (int i = 0; i < NB; i++) {
+            const int64_t k = c * NB + i;
+            if constexpr (OWN) {
+               u[i] += alpha * p[i];
+               r[i] -= alpha * q[i];
+            } else {
+               a.u[k] += alpha * p_now[k];
+               r[i] = a.r[k] - alpha * a.q[k];
+               a.r[k] = r[i];
+            }
+         }
+         d += precondition(c, r, z);
+#pragma unroll
+         for (int i = 0; i < NB; i++) a.z[c * NB + i] = z[i];
+      }
+      if (it + 1 == a.its) break;
+      double rho_new = 0.0;
+      if (!(ok = GridSum(d, a, step++, &rho_new))) break;
+      beta = rho != 0.0 ? rho_new / rho : 0.0;
+      rho = rho_new;
+   }
+   // A wait that gave up marks the solution, so that it is not taken for one
+   const double mark = __longlong_as_double(0x7ff8000000000000LL);
+   for (int64_t c = c0 + threadIdx.x; c < c1; c += kPcgThreads)
+#pragma unroll
+      for (int i = 0; i < NB; i++) {
+         if (!ok) a.u[c * NB + i] = mark;
+         else if (OWN) a.u[c * NB + i] = u[i];
+      }
 }
 
-// beta = rho_new / rho; p = z + beta p; rho = rho_new; clear rho_new and pq (one thread does the scalars)
-__global__ void CgDirectionKernel(int64_t n_nodes, const double *__restrict__ z, double *__restrict__ p, double *scal)
+template <int NB, int F, bool CSR>
+static int LaunchPcg(const DsaPcgArgs &args, cudaStream_t s)
 {
-   const int64_t node = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-   const double rho = scal[0], rho_new = scal[1];
-   const double beta = rho != 0.0 ? rho_new / rho : 0.0;
-   if (node < n_nodes) p[node] = z[node] + beta * p[node];
+   int dev = 0, sms = 0;
+   cudaGetDevice(&dev);
+   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+   const int64_t most = std::min<int64_t>((int64_t)sms * kPcgBlocksPerSm, 1024);
+   // As many cells per block as its threads, or as its shared memory holds
+   // where that still covers every cell with the blocks that run at once
+   constexpr int64_t kCellBytes = CSR ? 1 << 30 : KeptStride(F, NB) * (int64_t)sizeof(double);
+   const int64_t fit = std::min<int64_t>(kPcgThreads, kPcgKeepBytes / kCellBytes);
+   const bool keep = fit > 0 && args.n <= fit * most;
+   const int64_t want = keep ? (args.n + fit - 1) / fit : (args.n + kPcgThreads - 1) / kPcgThreads;
+   const int grid = (int)std::max<int64_t>(1, std::min(most, want));
+   const int64_t per = (args.n + grid - 1) / grid;
+   const bool own = per <= kPcgThreads;
+   auto kern = keep ? DsaPcgKernel<NB, F, CSR, true, !CSR>
+               : own ? DsaPcgKernel<NB, F, CSR, true, false> : DsaPcgKernel<NB, F, CSR, false, false>;
+   const size_t smem = keep ? (size_t)(per * kCellBytes) : 0;
+   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+   int rc = CudaCheck(cudaMemsetAsync(args.count, 0, sizeof(unsigned), s), "dsa solve");
+   if (rc) return rc;
+   DsaPcgArgs a = args;
+   void *params[] = {&a};
+   const cudaError_t e = cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(kPcgThreads), params, smem, s);
+   if (e != cudaSuccess) cudaGetLastError();
+   CountLaunch();
+   return CudaCheck(e, "dsa solve");
 }
 
-__global__ void CgRotateScalars(double *scal)
+// The inner solve on the given vectors, rhs restricted already (and overwritten)
+static int DsaPcg(const ubolt_ctx *ctx, const ubolt_dsa *ds, double *rhs, double *u, double *r, double *z, double *p,
+                  double *q, double *slots, cudaStream_t s)
 {
-   scal[0] = scal[1];
-   scal[1] = 0.0;
-   scal[2] = 0.0;
+   DsaPcgArgs a{};
+   a.n = ds->cg ? ds->n_nodes : ds->nc;
+   a.its = ds->inner_its;
+   a.code = ctx->g64.code;
+   a.rp = ds->d_rp;
+   a.col = ds->d_col;
+   a.val = ds->val;
+   a.jinv = ds->jinv;
+   a.rhs = rhs;
+   a.u = u;
+   a.r = r;
+   a.z = z;
+   a.p = p;
+   a.q = q;
+   a.count = reinterpret_cast<unsigned *>(slots);
+   a.slots = slots + 2;
+   if (ds->cg) return LaunchPcg<1, 1, true>(a, s);
+   UBOLT_DISPATCH(ds->nb, ds->F, return (LaunchPcg<NB_, F_, false>(a, s)));
+   return SetError(UBOLT_ERR_STATE, "no DSA kernel for this shape");
 }
 
 // ~~~ Host assembly
@@ -406,19 +574,25 @@ static int Assemble(ubolt_dsa *ds, const double *st, const double *ss)
    const size_t bs = (size_t)nb * nb;
    int rc = VoidPolicy(ds, st, ss);
    if (rc) return rc;
-   ds->h_val.assign(nc * (F + 1) * bs, 0.0);
-   ds->h_jinv.assign(nc * bs, 0.0);
+   ds->h_val.resize(nc * (F + 1) * bs);
+   ds->h_jinv.resize(nc * bs);
    const double *dcell = ds->h_d.data();
    const uint8_t *masked = ds->h_mask.data(), *is_void = ds->h_void.data();
 #pragma omp parallel for schedule(static)
    for (int64_t c = 0; c < nc; c++) {
-      double *blk = &ds->h_val[c * (F + 1) * bs];
+      double blk[(kMaxFaces + 1) * kMaxNb * kMaxNb] = {0.0}, inv[kMaxNb * kMaxNb];
       double *own = blk + F * bs;
       const double vol = ds->volume[c];
+      // Into the element-major stores
+      auto store = [&]() {
+         InvertSmall(nb, own, inv);
+         for (size_t k = 0; k < (F + 1) * bs; k++) ds->h_val[k * nc + c] = blk[k];
+         for (size_t k = 0; k < bs; k++) ds->h_jinv[k * nc + c] = inv[k];
+      };
       if (masked[c]) {
          // A masked void: V times the identity, every coupling zero
          for (int i = 0; i < nb; i++) own[i * nb + i] = vol;
-         InvertSmall(nb, own, &ds->h_jinv[c * bs]);
+         store();
          continue;
       }
       const double d_c = dcell[c];
@@ -500,7 +674,7 @@ static int Assemble(ubolt_dsa *ds, const double *st, const double *ss)
             }
          }
       }
-      InvertSmall(nb, own, &ds->h_jinv[c * bs]);
+      store();
    }
    return UBOLT_OK;
 }
@@ -563,21 +737,7 @@ static int AssembleCg(const ubolt_ctx *ctx, ubolt_dsa *ds, const double *st, con
 int DsaSolveOnDevice(ubolt_ctx *ctx, cudaStream_t s)
 {
    ubolt_dsa *ds = ctx->dsa;
-   const int64_t nn = ds->n_nodes;
-   const int bl = kDsaThreads;
-   const int64_t grid = (nn + bl - 1) / bl;
-   cudaMemsetAsync(ds->scal, 0, kDsaScalars * sizeof(double), s);
-   CgStartKernel<<<grid, bl, 0, s>>>(nn, ds->nb, ds->jinv, ds->rhs, ds->u, ds->r, ds->z, ds->p, ds->scal);
-   CountLaunch();
-   for (int it = 0; it < ds->inner_its; it++) {
-      DsaSpmvLaunch(ctx, ds, ds->p, ds->q, ds->p, ds->scal, s);
-      CgUpdateKernel<<<grid, bl, 0, s>>>(nn, ds->p, ds->q, ds->u, ds->r, ds->scal);
-      CgPrecondKernel<<<grid, bl, 0, s>>>(nn, ds->nb, ds->jinv, ds->r, ds->z, ds->scal);
-      CgDirectionKernel<<<grid, bl, 0, s>>>(nn, ds->z, ds->p, ds->scal);
-      CgRotateScalars<<<1, 1, 0, s>>>(ds->scal);
-      CountLaunch(5);
-   }
-   return CheckLaunch("dsa solve");
+   return DsaPcg(ctx, ds, ds->rhs, ds->u, ds->r, ds->z, ds->p, ds->q, ds->slots, s);
 }
 
 // The per-cell void mask of the current group, or NULL (no DSA filled, or no masked void)
@@ -627,7 +787,7 @@ void UboltDsaFree(ubolt_ctx *ctx)
    ubolt_dsa *ds = ctx->dsa;
    if (!ds) return;
    for (void *p : {(void *)ds->val, (void *)ds->jinv, (void *)ds->rhs, (void *)ds->u, (void *)ds->r, (void *)ds->z,
-                   (void *)ds->p, (void *)ds->q, (void *)ds->scal, (void *)ds->mask, (void *)ds->d_rp,
+                   (void *)ds->p, (void *)ds->q, (void *)ds->slots, (void *)ds->mask, (void *)ds->d_rp,
                    (void *)ds->d_col})
       if (p) cudaFree(p);
    delete ds;
@@ -649,6 +809,9 @@ extern "C" void ubolt_dsa_defaults(ubolt_dsa_options *o)
 
 // Device storage of one DSA: the operator's values (n_val), the Jacobi
 // inverses (n_jinv) and the inner solve's vectors and scalars
+// Blocks of one solve: never more than cells, nor than run at once
+static size_t PcgMostBlocks(size_t n) { return std::min<size_t>(n, 1024); }
+
 static int AllocDsa(ubolt_dsa *ds, size_t n_val, size_t n_jinv)
 {
    auto alloc = [&](double **p, size_t n) -> int {
@@ -663,7 +826,7 @@ static int AllocDsa(ubolt_dsa *ds, size_t n_val, size_t n_jinv)
    int rc = 0;
    if ((rc = alloc(&ds->val, n_val)) || (rc = alloc(&ds->jinv, n_jinv)) || (rc = alloc(&ds->rhs, nn)) ||
        (rc = alloc(&ds->u, nn)) || (rc = alloc(&ds->r, nn)) || (rc = alloc(&ds->z, nn)) || (rc = alloc(&ds->p, nn)) ||
-       (rc = alloc(&ds->q, nn)) || (rc = alloc(&ds->scal, kDsaScalars + (nn + kDsaThreads - 1) / kDsaThreads)))
+       (rc = alloc(&ds->q, nn)) || (rc = alloc(&ds->slots, 2 + 2 * PcgMostBlocks(nn))))
       return rc;
    return UBOLT_OK;
 }
@@ -877,8 +1040,7 @@ extern "C" int ubolt_dsa_spmv(ubolt_ctx *ctx, const double *u, double *v, void *
    int rc = CheckReady(ctx, false);
    if (rc || (rc = CheckDsa(ctx))) return rc;
    if (!u || !v || u == v) return SetError(UBOLT_ERR_ARG, "dsa_spmv: u and v must be distinct device arrays");
-   DsaSpmvLaunch(ctx, ctx->dsa, u, v, nullptr, nullptr, (cudaStream_t)stream);
-   return CheckLaunch("dsa_spmv");
+   return DsaSpmvLaunch(ctx, ctx->dsa, u, v, (cudaStream_t)stream);
 }
 
 extern "C" int ubolt_dsa_restrict(ubolt_ctx *ctx, const double *x, double *rhs, void *stream)
@@ -923,7 +1085,10 @@ extern "C" int ubolt_dsa_matrix(ubolt_ctx *ctx, double *blocks)
    if (rc || (rc = CheckDsa(ctx))) return rc;
    if (!blocks) return SetError(UBOLT_ERR_ARG, "dsa_matrix: NULL output");
    if (ctx->dsa->cg) return SetError(UBOLT_ERR_STATE, "dsa_matrix: the CG-SUPG operator is CSR, read it by ubolt_dsa_spmv");
-   std::copy(ctx->dsa->h_val.begin(), ctx->dsa->h_val.end(), blocks);
+   const ubolt_dsa *ds = ctx->dsa;
+   const size_t per = (size_t)(ds->F + 1) * ds->nb * ds->nb;
+   for (int64_t c = 0; c < ds->nc; c++)
+      for (size_t k = 0; k < per; k++) blocks[c * per + k] = ds->h_val[k * ds->nc + c];
    return UBOLT_OK;
 }
 
@@ -940,9 +1105,9 @@ extern "C" int ubolt_dsa_matrix(ubolt_ctx *ctx, double *blocks)
 namespace {
 
 // Six node vectors (restricted rhs and the PCG's u, r, z, p, q) of at most
-// kStaticDsaNodes nodes each, then the scalars and one partial sum per block
+// kStaticDsaNodes nodes each, then the grid sums' counter and slots
 constexpr int64_t kStaticDsaNodes = (int64_t)1 << 18;
-constexpr int64_t kStaticDsaDoubles = 6 * kStaticDsaNodes + kDsaScalars + kStaticDsaNodes / kDsaThreads;
+constexpr int64_t kStaticDsaDoubles = 6 * kStaticDsaNodes + 2 + 2 * 1024;
 static __device__ __align__(256) double g_dsa_scratch[kStaticDsaDoubles];
 
 constexpr int kMaxDevices = 64;
@@ -983,26 +1148,13 @@ extern "C" int ubolt_dsa_apply_static(ubolt_ctx *ctx, const double *x, double *y
    if ((rc = StaticScratch(ctx->device, &base))) return rc;
    const int64_t nn = kStaticDsaNodes;
    double *rhs = base, *u = base + nn, *r = base + 2 * nn, *z = base + 3 * nn, *p = base + 4 * nn, *q = base + 5 * nn;
-   double *scal = base + 6 * nn;
+   double *slots = base + 6 * nn;
    cudaStream_t s = (cudaStream_t)stream;
    DsaRestrictKernel<double><<<RunGrid(ds->n_nodes), 256, 0, s>>>(ds->n_nodes, ds->nb, ctx->A, ctx->geom<double>().w,
                                                                    ctx->d_volume, x, nullptr, ds->mask, rhs);
    CountLaunch();
-   // The same fixed-count block-Jacobi PCG as the workspace path; the
-   // scalars are cleared here, every vector is written before it is read
-   const int64_t nodes = ds->n_nodes;
-   const int64_t grid = (nodes + 255) / 256;
-   if ((rc = CudaCheck(cudaMemsetAsync(scal, 0, kDsaScalars * sizeof(double), s), "dsa_apply_static"))) return rc;
-   CgStartKernel<<<grid, 256, 0, s>>>(nodes, ds->nb, ds->jinv, rhs, u, r, z, p, scal);
-   CountLaunch();
-   for (int it = 0; it < ds->inner_its; it++) {
-      DsaSpmvLaunch(ctx, ds, p, q, p, scal, s);
-      CgUpdateKernel<<<grid, 256, 0, s>>>(nodes, p, q, u, r, scal);
-      CgPrecondKernel<<<grid, 256, 0, s>>>(nodes, ds->nb, ds->jinv, r, z, scal);
-      CgDirectionKernel<<<grid, 256, 0, s>>>(nodes, z, p, scal);
-      CgRotateScalars<<<1, 1, 0, s>>>(scal);
-      CountLaunch(5);
-   }
+   // The same solve as the workspace path's; every vector is written before it is read
+   if ((rc = DsaPcg(ctx, ds, rhs, u, r, z, p, q, slots, s))) return rc;
    DsaProlongKernel<double><<<RunGrid(ctx->n_nodes), 256, 0, s>>>(ctx->n_nodes, ds->nb, ctx->A,
                                                                       1.0 / ctx->sum_weights, u, ds->mask, y, 0);
    return CheckLaunch("dsa_apply_static");
