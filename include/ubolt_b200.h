@@ -338,14 +338,12 @@ typedef struct {
  * streamed in by bulk copies - meshes whose every ordinate's upwind graph is
  * acyclic (2D, hexahedra), with a reserved factor store, no wait on another
  * block. One block per ordinate leaves most SMs idle and pays for every
- * scattered psi word on one SM, so AUTO picks WAVE only where it applies
- * and the problem is small (n_cells A <= 2^17, where it measured faster),
- * TASKS otherwise. */
+ * scattered psi word on one SM; TASKS measured faster at every size, and AUTO
+ * is TASKS. */
 enum { UBOLT_SWEEP_AUTO = 0, UBOLT_SWEEP_TASKS = 1, UBOLT_SWEEP_WAVE = 2 };
 
-/* Build the sweep plan: patches of patch_size consecutive cells (0 picks 64,
- * or 48 on tetrahedra;
- * at most 256), per-ordinate upwind orders, task list; then reserve the
+/* Build the sweep plan: patches of patch_size consecutive cells (0 picks
+ * 48 to 256 by shape, order and size; at most 256), per-ordinate upwind orders, task list; then reserve the
  * factor stores and one scratch vector (see ubolt_sweep_set_factor_limit). Host work, one upload
  * and the sweep's only device allocations; independent of the group.
  * Called by the first sweep if not before. The streaming stage of the preconditioner, in place of

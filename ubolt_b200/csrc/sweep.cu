@@ -57,18 +57,29 @@ constexpr int kCtrlCounter = 0, kCtrlError = ubolt::kSweepCtrlError, kCtrlNever 
 constexpr int kSweepWarpsPerSm = 32;
 constexpr size_t kViaBytes = (size_t)8 << 20;
 constexpr uint32_t kCopyTries = 1u << 22;  // bounded wait for a task's bulk copy
-constexpr int kDefaultPatch = 64;
 
-// The default patch: half a tile of the mesh builders' cell numbering (8 x 8
-// quads, 4^3 hexes), and eight cubes' worth of Kuhn tetrahedra. Measured per
-// isotropic-source sweep at S8 (FP64 / FP32, us): 256^2 triangles 595 / 488 at
-// 64 cells, 607 / 418 at 128, 921 / 813 at 32; 200^2 quadrilaterals 301 / 268
-// at 64, 354 / 312 at 32, 312 / 263 at 128; 20^3 cubes of Kuhn tetrahedra 901 /
-// 492 at 48, 946 / 673 at 24, 1361 / 599 at 96; 40^3 hexahedra 603 / 399 at 64,
-// 683 / 350 at 32
+// The default patch, in cells. Larger patches make fewer and longer tasks
+// with fewer waits between them, but their couplings take the shared memory of
+// resident warps, and a task starts as late as its latest ghost. Measured per
+// isotropic-source sweep at S8 (FP64 / FP32, us), a multiple or a part of the
+// mesh builders' tiles (8 x 8 quads, 4^3 boxes) best:
+//    256^2 triangles DG1     64: 591 / 485    128: 602 / 415    32: 921 / 813
+//    100^2 quads DG1         64: 150 / 136    128: 139 / 124
+//    101 x 77 triangles DG1  64: 154 / 142    128: 142 / 135
+//    20^3 cubes of tets DG1  48: 901 / 492    24: 946 / 673     96: 1361 / 599
+//    40^3 hexes DG1          64: 603 / 399    32: 683 / 350
+// and DG0, whose couplings are one value each:
+//    150^2 triangles         64: 256 / 237    256: 197 / 183
+//    200^2 quads             64: 234 / 221    256: 225 / 212
+//    20^3 cubes of tets      48: 386 / 351    192: 213 / 196
+//    40^3 hexes              64: 150 / 136    128: 129 / 115    256: 155 / 125
 static int DefaultPatch(const ubolt_ctx *ctx)
 {
-   return (ctx->dim == 3 && ctx->F == 4) ? 48 : kDefaultPatch;
+   const bool tets = ctx->dim == 3 && ctx->F == 4;
+   if (ctx->nb == 1) return ctx->dim == 2 ? 256 : tets ? 192 : 128;
+   if (ctx->dim == 3) return tets ? 48 : 64;
+   // Few cell-ordinates fill the device with tasks of either size
+   return ctx->n_cells * (int64_t)ctx->A <= (int64_t)1 << 20 ? 128 : 64;
 }
 
 namespace ubolt {
@@ -104,7 +115,7 @@ struct ubolt_sweep_plan {
    // graph is acyclic and a level fits a block: wave[which].smem > 0 where
    // precision `which` (0 FP64, 1 FP32) can run it. fac_wave[which]: the
    // store reserved for that precision is in wave order (the wave kernel runs)
-   bool wave_ok = false;
+   bool wave_tried = false, wave_ok = false;  // built when the wave kernel is asked for
    int wave_threads = 256;
    int64_t wave_levels = 0;
    ubolt::WaveDev wave[2];
@@ -719,6 +730,8 @@ static int SweepSlots(int F, int max_inflow)
 // upwind cycle or a level or front too large for one block.
 static int BuildWavePlan(ubolt_ctx *ctx, ubolt_sweep_plan *plan)
 {
+   if (plan->wave_tried) return UBOLT_OK;
+   plan->wave_tried = true;
    HostWavePlan h;
    BuildHostWavePlan(ctx->n_cells, ctx->F, ctx->A, ctx->h_omega.data(), ctx->h_nA.data(), ctx->h_code.data(), h);
    if (!h.acyclic || h.S > std::min(4, ctx->F - 1) || h.n_slots >= 0xffff || h.max_width > 512) return UBOLT_OK;
@@ -892,12 +905,14 @@ int BuildSweepPlan(ubolt_ctx *ctx, int patch_size)
    plan->ctrl = static_cast<uint32_t *>(p);
    cudaMemset(plan->ctrl, 0, kCtrlWords * sizeof(uint32_t));
    cudaMemset(plan->ctrl + kCtrlNever, 0xff, 2 * sizeof(uint32_t));
-   if ((rc = BuildWavePlan(ctx, plan))) { delete plan; return rc; }
    if (ctx->sweep) {
       plan->fac_limit = ctx->sweep->fac_limit;
       plan->kernel_mode = ctx->sweep->kernel_mode;
    }
-   if (plan->kernel_mode == UBOLT_SWEEP_WAVE && !plan->wave_ok) plan->kernel_mode = UBOLT_SWEEP_AUTO;
+   if (plan->kernel_mode == UBOLT_SWEEP_WAVE) {
+      if ((rc = BuildWavePlan(ctx, plan))) { delete plan; return rc; }
+      if (!plan->wave_ok) plan->kernel_mode = UBOLT_SWEEP_AUTO;
+   }
    delete ctx->sweep;
    ctx->sweep = plan;
    if ((rc = CudaCheck(cudaDeviceSynchronize(), "sweep plan"))) return rc;
@@ -1008,14 +1023,6 @@ static int64_t FactorBytes(const ubolt_ctx *ctx, const ubolt_sweep_plan *pl, siz
 // half the free device memory at that moment (at most 96 GiB); 0: none;
 // otherwise the byte limit for both together. A store not reserved means
 // the sweep computes its factors as it goes: the result is the same.
-// The automatic choice. The wave kernel runs one block per ordinate, and a
-// block's level costs about one L1 wavefront per scattered q and psi word:
-// on one B200 it beat the task kernel only on small problems (64^2 quads
-// DG0 S4: 0.078 against 0.110 ms) and lost from 128^2 triangles DG1 S8
-// (0.77 against 0.39 ms) up to 256^2 at S16 (3.78 against 3.71 ms). So it is
-// taken up to 2^17 cell-ordinates.
-static bool WavePreferred(const ubolt_ctx *ctx) { return ctx->n_cells * (int64_t)ctx->A <= ((int64_t)1 << 17); }
-
 static int ReserveFactors(ubolt_ctx *ctx, int64_t limit)
 {
    ubolt_sweep_plan *pl = ctx->sweep;
@@ -1037,10 +1044,13 @@ static int ReserveFactors(ubolt_ctx *ctx, int64_t limit)
    }
    int64_t left = limit;
    for (int which : {1, 0}) {
-      // The wave kernel where it applies and is chosen (its store is in wave
-      // order), else the task kernel's
-      const bool wave = pl->wave[which].smem > 0 &&
-                        (pl->kernel_mode == UBOLT_SWEEP_WAVE || (pl->kernel_mode == UBOLT_SWEEP_AUTO && WavePreferred(ctx)));
+      // The wave kernel's store is in wave order. It runs where it is asked
+      // for: one block per ordinate leaves most of the device idle, and the
+      // task kernel was faster on every mesh measured (FP64, us, wave and
+      // tasks: 64^2 quads DG0 S4 68 / 41, 32^2 37 / 23, 24^2 triangles DG1 S8
+      // 84 / 38, 16^3 hexes DG1 S2 72 / 53, 8^3 hexes DG1 S4 27 / 25, 256^2
+      // triangles DG1 S8 2220 / 703)
+      const bool wave = pl->wave[which].smem > 0 && pl->kernel_mode == UBOLT_SWEEP_WAVE;
       pl->fac_wave[which] = false;
       const int64_t bytes = wave ? pl->wave_bytes[which] : FactorBytes(ctx, pl, which ? 4 : 8);
       if (bytes > left) continue;
@@ -1279,6 +1289,7 @@ extern "C" int ubolt_sweep_set_kernel(ubolt_ctx *ctx, int kernel)
    if (kernel < UBOLT_SWEEP_AUTO || kernel > UBOLT_SWEEP_WAVE) return SetError(UBOLT_ERR_ARG, "sweep kernel %d", kernel);
    if (!ctx->sweep && (rc = BuildSweepPlan(ctx, 0))) return rc;
    ubolt_sweep_plan *pl = ctx->sweep;
+   if (kernel == UBOLT_SWEEP_WAVE && (rc = BuildWavePlan(ctx, pl))) return rc;
    if (kernel == UBOLT_SWEEP_WAVE && !pl->wave_ok)
       return SetError(UBOLT_ERR_STATE, "the wave sweep does not apply here (an upwind cycle, or a level or front too "
                                        "large for one block)");
