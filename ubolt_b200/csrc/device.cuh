@@ -440,6 +440,22 @@ __device__ __forceinline__ bool CellFactors(const DevGeom<T> &g, int64_t c, cons
    return ok;
 }
 
+// A grid barrier's arrival and wait, by one thread of a block of a cooperative
+// launch: the block's writes so far are released, `target` arrivals waited for
+// (the blocks' number times the barriers so far), the others' writes acquired.
+// Bounded; false: gave up. The fence empties the SM's L1.
+__device__ __forceinline__ bool GridArrive(unsigned *count, unsigned target)
+{
+   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+   unsigned v;
+   uint32_t tries = 0;
+   do {
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+   } while ((int)(v - target) < 0 && ++tries < (1u << 24));
+   __threadfence();
+   return (int)(v - target) >= 0;
+}
+
 // Node-run kernels. A node's A ordinates are one contiguous run of psi. A
 // warp takes kLpn = 8 lanes per node, four nodes at a time; lane `sub` of a
 // node strides its run by 8, so every load or store of the warp covers four

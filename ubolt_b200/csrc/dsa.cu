@@ -79,10 +79,9 @@ struct ubolt_dsa {
 namespace ubolt {
 
 // The PCG's blocks: one of 512 threads per SM (at two of 384 the kernel
-// spilled, and a spill is a trip to L2 here, as every grid sum empties L1), the
-// tries of a bounded wait, and the shared memory a block may hold of the matrix
+// spilled, and a spill is a trip to L2 here, as every grid sum empties L1), and the
+// shared memory a block may hold of the matrix
 constexpr int kPcgThreads = 512, kPcgBlocksPerSm = 1;
-constexpr uint32_t kPcgTries = 1u << 24;
 constexpr int64_t kPcgKeepBytes = 220 * 1024;
 // A cell's matrix in shared memory, an odd number of values apart (no bank conflicts)
 __host__ __device__ constexpr int KeptStride(int F, int NB) { return (F + 1) * NB * NB | 1; }
@@ -248,16 +247,8 @@ __device__ __forceinline__ bool GridSum(double d, const DsaPcgArgs &a, unsigned 
 #pragma unroll
          for (int w = 0; w < kWarps; w++) s += red[w];
          row[blockIdx.x] = s;
-         // The block's writes of this phase before its arrival (its threads met above)
-         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.count) : "memory");
-         const unsigned target = (step + 1) * (unsigned)G;
-         unsigned v;
-         uint32_t tries = 0;
-         do {
-            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.count) : "memory");
-         } while (v < target && ++tries < kPcgTries);
-         ok = v >= target;
-         __threadfence();
+         // (the block's threads met above: their writes of this phase are released too)
+         ok = GridArrive(a.count, (step + 1) * (unsigned)G);
       }
       __syncwarp();
       double t = 0.0;

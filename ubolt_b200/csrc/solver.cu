@@ -52,8 +52,10 @@ struct ubolt_solver {
    float *Z32 = nullptr;
    // Reductions: partial[red_blocks][restart + 2], h[3 * (restart + 2)]
    double *partial = nullptr, *h = nullptr;
-   int red_blocks = 0;
-   unsigned *md_count = nullptr;  // the multi-dot's finished-block counter, zero between launches
+   int red_blocks = 0, gs_blocks = 0;
+   // [0] the multi-dot's finished-block counter, zero between launches; [1] the
+   // Gram-Schmidt kernel's barrier counter
+   unsigned *md_count = nullptr;
    // The compressed form (sweep preconditioner, exact sweep): node-space
    // basis (restart + 1) x n_nodes, the residual's isotropic part, the basis
    // scalars alpha[restart + 2] and four reduction slots
@@ -79,71 +81,154 @@ namespace ubolt {
 constexpr int kRedThreads = 256;
 constexpr int kChunk = 8;
 
-// One Gram-Schmidt pass's scalars of the compressed basis, formed by the
-// multi-dot's last block once every dot is in (see IsoCombine below)
-struct IsoCombineArgs {
-   double *alpha = nullptr;
-   int j1 = 0, first = 0, on = 0;
-   double rp2 = 0.0, kappa = 0.0;
+// The Gram-Schmidt step of the compressed basis in one cooperative launch:
+// two classical passes over the node vectors, the new vector's norm and its
+// scaling, with a grid barrier after each reduction. In the inner product of
+// the compressed form,
+//    h_i = alpha_i alpha_w |r_perp|^2 + kappa <phi_i, phi_w>,
+//    alpha_w -= sum_i h_i alpha_i,  phi_w -= sum_i h_i phi_i,
+// alpha_w starting as the last vector's scalar; then hn = sqrt(alpha_w^2
+// |r_perp|^2 + kappa |phi_w|^2), and where it is positive and finite alpha_w
+// and phi_w are divided by it (else left; the host sees the same hn and
+// stops). The two passes' h, |phi_w|^2 and alpha_w before the division go to
+// the mailbox, from which the host forms the Hessenberg column. Every block
+// adds all blocks' shares itself, in one order, so all hold the same scalars.
+// Bound by the barriers (about 2 us each with the sums) and, for long vectors, by
+// 4 (j + 2) n_nodes 8 bytes through L2. As eight launches a step (dots, updates,
+// scaling) 256^2 triangles (393 k nodes) took about 60 us, now 34; a whole solve
+// of 64^2 DG0 quadrilaterals (8 steps) 870 -> 709 us, of 256^2 triangles 5.54 ->
+// 5.37 ms.
+constexpr int kGsThreads = 512, kGsBlocksPerSm = 2;
+constexpr int kGsMost = 201;  // basis vectors: the longest restart and one
+
+struct GsArgs {
+   const double *Phi;  // [j1][n]
+   double *w;          // [n]: in phi_w, out the new basis vector
+   int64_t n;
+   int j1;
+   double *alpha;  // [j1 + 1]; [j1] written
+   double rp2, kappa;
+   double *partial;  // [blocks][stride]
+   int stride;
+   unsigned *count;
+   unsigned base;  // the counter's value at launch
+   double *box_h1, *box_h2, *box_alpha;  // mailbox: h1[j1], h2[j1 + 1] (last |phi_w|^2), alpha_w
 };
 
-// h[i] = alpha[i] alpha_w |r_perp|^2 + kappa d[i] for i < j1 (in place over
-// d), then alpha[j1] = alpha_w - sum_i h[i] alpha[i]: one Gram-Schmidt
-// pass's scalars. alpha_w is alpha[j1], or on the first pass alpha[j1 - 1]
-// (the new vector w = v_j - ... starts with v_j's scalar). One thread.
-__device__ __forceinline__ void IsoCombine(double *__restrict__ d, const IsoCombineArgs &c)
+__global__ void __launch_bounds__(kGsThreads, kGsBlocksPerSm) GramSchmidtKernel(const GsArgs a)
 {
-   double *alpha = c.alpha;
-   const int j1 = c.j1;
-   const double aw = c.first ? alpha[j1 - 1] : alpha[j1];
-   double upd = 0.0;
-   for (int i = 0; i < j1; i++) {
-      const double h = alpha[i] * aw * c.rp2 + c.kappa * d[i];
-      d[i] = h;
-      upd += h * alpha[i];
+   constexpr int kWarps = kGsThreads / 32;
+   __shared__ double h[kGsMost], al[kGsMost], red[kChunk][kWarps];
+   __shared__ double aw, scale;
+   __shared__ int ok;
+   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, G = gridDim.x, j1 = a.j1;
+   const int64_t first = (int64_t)blockIdx.x * kGsThreads + t, step = (int64_t)G * kGsThreads;
+   unsigned barriers = 0;
+   for (int i = t; i < j1; i += kGsThreads) al[i] = a.alpha[i];
+   if (t == 0) ok = 1;
+   __syncthreads();
+   if (t == 0) aw = al[j1 - 1];
+   // h[i] = the sum over the grid of every block's share of value i
+   auto grid_sum = [&](int n_values) {
+      __syncthreads();
+      if (t == 0) ok = GridArrive(a.count, a.base + ++barriers * (unsigned)G) && ok;
+      __syncthreads();
+      for (int i = warp; i < n_values; i += kWarps) {
+         double s = 0.0;
+         for (int b = lane; b < G; b += 32) s += __ldcg(a.partial + (int64_t)b * a.stride + i);
+#pragma unroll
+         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+         if (lane == 0) h[i] = s;
+      }
+      __syncthreads();
+   };
+   // The block's shares of nc values held by its threads, from value i0
+   auto share = [&](double (&acc)[kChunk], int i0, int nc) {
+#pragma unroll
+      for (int i = 0; i < kChunk; i++) {
+         double v = acc[i];
+#pragma unroll
+         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+         if (lane == 0) red[i][warp] = v;
+      }
+      __syncthreads();
+      if (t < nc) {
+         double s = 0.0;
+         for (int w = 0; w < kWarps; w++) s += red[t][w];
+         a.partial[(int64_t)blockIdx.x * a.stride + i0 + t] = s;
+      }
+      __syncthreads();
+   };
+   for (int pass = 0; pass < 2; pass++) {
+      for (int i0 = 0; i0 < j1; i0 += kChunk) {
+         const int nc = min(kChunk, j1 - i0);
+         double acc[kChunk];
+#pragma unroll
+         for (int i = 0; i < kChunk; i++) acc[i] = 0.0;
+         for (int64_t k = first; k < a.n; k += step) {
+            const double wk = a.w[k];
+#pragma unroll
+            for (int i = 0; i < kChunk; i++)
+               if (i < nc) acc[i] += __ldg(a.Phi + (int64_t)(i0 + i) * a.n + k) * wk;
+         }
+         share(acc, i0, nc);
+      }
+      grid_sum(j1);
+      // The pass's scalars (one warp: the sum in lane order, the same everywhere)
+      if (warp == 0) {
+         double upd = 0.0;
+         for (int i = lane; i < j1; i += 32) {
+            const double hv = al[i] * aw * a.rp2 + a.kappa * h[i];
+            upd += hv * al[i];
+            h[i] = hv;
+            if (blockIdx.x == 0) (pass ? a.box_h2 : a.box_h1)[i] = hv;
+         }
+#pragma unroll
+         for (int o = 16; o > 0; o >>= 1) upd += __shfl_xor_sync(0xffffffffu, upd, o);
+         if (lane == 0) aw -= upd;
+      }
+      __syncthreads();
+      double norm = 0.0;
+      for (int64_t k = first; k < a.n; k += step) {
+         double wk = a.w[k];
+#pragma unroll 4
+         for (int i = 0; i < j1; i++) wk -= h[i] * __ldg(a.Phi + (int64_t)i * a.n + k);
+         a.w[k] = wk;
+         norm += wk * wk;
+      }
+      if (pass == 1) {
+         double acc[kChunk] = {norm};
+         share(acc, 0, 1);
+      }
    }
-   alpha[j1] = aw - upd;
-}
-
-// The new Arnoldi vector's norm from its two parts, hn = sqrt(alpha_w^2
-// |r_perp|^2 + kappa |phi_w|^2); where it is positive and finite, alpha[j1]
-// = alpha_w / hn and inv[0] = 1 / hn, else inv[0] = 1 (the vector is left as
-// it is; the host sees the same hn and stops). The host forms the same hn
-// from the same values for the Hessenberg column.
-__global__ void IsoNormalizeKernel(const double *__restrict__ phi2, double *__restrict__ alpha, int j1, double rp2,
-                                   double kappa, double *__restrict__ inv)
-{
-   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-   const double aw = alpha[j1];
-   // Rounded step by step (no fused multiply-add), as the host's expression is
-   const double hn = sqrt(__dadd_rn(__dmul_rn(__dmul_rn(aw, aw), rp2), __dmul_rn(kappa, phi2[0])));
-   if (hn > 0.0 && isfinite(hn)) {
-      alpha[j1] = aw / hn;
-      inv[0] = 1.0 / hn;
-   } else {
-      inv[0] = 1.0;
+   grid_sum(1);
+   if (t == 0) {
+      const double phi2 = ok ? h[0] : __longlong_as_double(0x7ff8000000000000LL);  // gave up: the host stops
+      // Rounded step by step (no fused multiply-add), as the host's expression is
+      const double hn = sqrt(__dadd_rn(__dmul_rn(__dmul_rn(aw, aw), a.rp2), __dmul_rn(a.kappa, phi2)));
+      const bool good = hn > 0.0 && isfinite(hn);
+      scale = good ? 1.0 / hn : 1.0;
+      if (blockIdx.x == 0) {
+         a.box_h2[j1] = phi2;
+         a.box_alpha[0] = aw;
+         a.alpha[j1] = good ? aw / hn : aw;
+      }
    }
-}
-
-// x *= s[0], s on the device
-__global__ void ScaleByDeviceKernel(double *__restrict__ x, const double *__restrict__ sp, int64_t n)
-{
-   const double sc = sp[0];
-   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-      x[k] = sc * x[k];
+   __syncthreads();
+   const double sc = scale;
+   for (int64_t k = first; k < a.n; k += step) a.w[k] = sc * a.w[k];
 }
 
 // h[i0 + i] = V_{i0+i} . w for i < nc: each block's share to
 // partial[blk][i0 + i], then the last block to finish (an integer counter,
 // reset by that block) adds the shares in a fixed order, one warp per value:
 // per-lane strided sums, then a shuffle tree, the same every run. No block
-// waits on another. With cmb.on (the last chunk of a compressed-basis pass)
-// that block then forms the pass's scalars from all of h.
+// waits on another.
 template <typename S>
 __global__ void __launch_bounds__(kRedThreads) MultiDotKernel(const S *__restrict__ V, int64_t n, int i0, int nc,
                                                               const S *__restrict__ w, double *__restrict__ partial,
                                                               int stride, double *__restrict__ h,
-                                                              unsigned *__restrict__ count, IsoCombineArgs cmb)
+                                                              unsigned *__restrict__ count)
 {
    double acc[kChunk];
 #pragma unroll
@@ -184,10 +269,6 @@ __global__ void __launch_bounds__(kRedThreads) MultiDotKernel(const S *__restric
       if (lane == 0) h[i0 + warp] = s;
    }
    if (threadIdx.x == 0) *count = 0;
-   if (cmb.on) {
-      __syncthreads();
-      if (threadIdx.x == 0) IsoCombine(h, cmb);
-   }
 }
 
 // out[i] = sum over blocks of partial[blk][i]
@@ -256,18 +337,15 @@ static int GridFor(int64_t n)
 
 // h[0..nv) = V^T w, computed on the device
 template <typename S>
-static void MultiDot(const ubolt_solver *ws, const S *V, int nv, const S *w, int64_t n, double *h, cudaStream_t s,
-                     IsoCombineArgs cmb = IsoCombineArgs())
+static void MultiDot(const ubolt_solver *ws, const S *V, int nv, const S *w, int64_t n, double *h, cudaStream_t s)
 {
    const int stride = ws->restart + 2;
    // Four elements per thread: a short (node-space) vector still spreads
    // over a few hundred blocks, and the partials to reduce stay few
    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(ws->red_blocks, n / (4 * kRedThreads)));
    for (int i0 = 0; i0 < nv; i0 += kChunk) {
-      IsoCombineArgs c = cmb;
-      c.on = cmb.on && i0 + kChunk >= nv;  // after the last chunk's dots
       MultiDotKernel<S><<<blocks, kRedThreads, 0, s>>>(V, n, i0, std::min(kChunk, nv - i0), w, ws->partial, stride,
-                                                       h, ws->md_count, c);
+                                                       h, ws->md_count);
    }
    CountLaunch((nv + kChunk - 1) / kChunk);
 }
@@ -331,6 +409,42 @@ static void ToDevice(const ubolt_solver *ws, const double *host, double *dev, in
    for (int i = 0; i < n; i++) box[i] = host[i];
    MailCopyKernel<<<1, 64, 0, s>>>(ws->mb_d + ws->mb_half + off, dev, n);
    CountLaunch();
+}
+
+// One Gram-Schmidt step of the compressed basis (see GramSchmidtKernel): w
+// against Phi[0 .. j1), scalars in alpha, the Hessenberg column to the mailbox.
+// *base: the barrier counter's value, advanced by the launch's arrivals.
+static int GramSchmidt(const ubolt_solver *ws, const double *Phi, int j1, double *w, double *alpha, double rp2,
+                       double kappa, unsigned *base, cudaStream_t s)
+{
+   int dev = 0, sms = 0, per_sm = 0;
+   cudaGetDevice(&dev);
+   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, GramSchmidtKernel, kGsThreads, 0);
+   const int64_t most = std::min<int64_t>((int64_t)sms * std::max(1, std::min(per_sm, kGsBlocksPerSm)), ws->gs_blocks);
+   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(most, (ws->n_nodes + kGsThreads - 1) / kGsThreads));
+   GsArgs a{};
+   a.Phi = Phi;
+   a.w = w;
+   a.n = ws->n_nodes;
+   a.j1 = j1;
+   a.alpha = alpha;
+   a.rp2 = rp2;
+   a.kappa = kappa;
+   a.partial = ws->partial;
+   a.stride = ws->restart + 2;
+   a.count = ws->md_count + 1;
+   a.base = *base;
+   a.box_h1 = ws->mb_d + kMbH1;
+   a.box_h2 = ws->mb_d + kMbH1 + (ws->restart + 2);
+   a.box_alpha = ws->mb_d + kMbScalars;
+   void *params[] = {&a};
+   const cudaError_t e = cudaLaunchCooperativeKernel((const void *)GramSchmidtKernel, dim3(grid), dim3(kGsThreads), params,
+                                                     0, s);
+   if (e != cudaSuccess) cudaGetLastError();
+   *base += 3u * (unsigned)grid;
+   CountLaunch();
+   return CudaCheck(e, "gram-schmidt");
 }
 
 template <typename S>
@@ -816,8 +930,11 @@ static int GmresIso(ubolt_ctx *ctx, const ubolt_solver *ws, S *work, const S *b,
    double *Phi = ws->Phi, *alpha = ws->alpha, *scal = ws->scal;
    std::vector<double> H((size_t)(m + 1) * m, 0.0), cs(m), sn(m), gv(m + 1), y(m), h1(m + 1), h2(m + 2),
        alpha_h(m + 2, 0.0);
-   double *dh1 = ws->h, *dh2 = ws->h + (m + 2), *dy = ws->h + 2 * (m + 2);
+   double *dy = ws->h + 2 * (m + 2);
    int rc = 0;
+   // The Gram-Schmidt kernel's barrier counter starts every system at zero
+   unsigned gs_base = 0;
+   if ((rc = CudaCheck(cudaMemsetAsync(ws->md_count + 1, 0, sizeof(unsigned), s), "gmres"))) return rc;
    out->iterations = 0;
    out->converged = false;
    while (out->iterations < max_it) {
@@ -875,27 +992,10 @@ static int GmresIso(ubolt_ctx *ctx, const ubolt_solver *ws, S *work, const S *b,
          else
             IsoScatterKernel<S><<<igrid, 256, 0, s>>>(z, wgt, sig_s, 1.0 / ctx->sum_weights, ctx->nb, A, nn, pj, pn);
          CountLaunch();
-         // Classical Gram-Schmidt, twice, in the compressed inner product
-         for (int pass = 0; pass < 2; pass++) {
-            double *dh = pass ? dh2 : dh1;
-            IsoCombineArgs cmb;
-            cmb.alpha = alpha;
-            cmb.j1 = j + 1;
-            cmb.first = pass == 0;
-            cmb.on = 1;
-            cmb.rp2 = rp2;
-            cmb.kappa = kappa;
-            MultiDot<double>(ws, Phi, j + 1, pn, nn, dh, s, cmb);
-            MultiAxpyKernel<double><<<igrid, 256, 0, s>>>(Phi, nn, j + 1, dh, -1.0, pn, 1);
-            CountLaunch();
-         }
-         MultiDot<double>(ws, pn, 1, pn, nn, dh2 + j + 1, s);
-         ToHost3(ws, MailRuns{{dh1, dh2, alpha + j + 1}, {kMbH1, kMbH1 + (m + 2), kMbScalars}, {j + 1, j + 2, 1}}, s);
-         // The new vector normalised on the device, behind the mailbox
-         // copy, so that the next sweep waits on nothing the host sends
-         IsoNormalizeKernel<<<1, 32, 0, s>>>(dh2 + j + 1, alpha, j + 1, rp2, kappa, scal + 3);
-         ScaleByDeviceKernel<<<igrid, 256, 0, s>>>(pn, scal + 3, nn);
-         CountLaunch(2);
+         // Classical Gram-Schmidt, twice, in the compressed inner product, and
+         // the new vector normalised on the device, so that the next sweep
+         // waits on nothing the host sends
+         if ((rc = GramSchmidt(ws, Phi, j + 1, pn, alpha, rp2, kappa, &gs_base, s))) return rc;
          if ((rc = CudaCheck(cudaStreamSynchronize(s), "gmres"))) return rc;
          std::copy(ws->mb_h + kMbH1, ws->mb_h + kMbH1 + j + 1, h1.begin());
          std::copy(ws->mb_h + kMbH1 + (m + 2), ws->mb_h + kMbH1 + (m + 2) + j + 2, h2.begin());
@@ -980,6 +1080,7 @@ static int EnsureWorkspace(ubolt_ctx *ctx, const ubolt_solve_options *o)
    ws->mixed = mixed;
    ws->flexible = flexible;
    ws->red_blocks = std::min(GridFor(ws->n), 1184);
+   ws->gs_blocks = 512;
    const int64_t n = ws->n;
    auto alloc = [&](void **p, size_t bytes) -> int {
       const cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
@@ -994,7 +1095,7 @@ static int EnsureWorkspace(ubolt_ctx *ctx, const ubolt_solve_options *o)
    int rc = 0;
    ctx->solver = ws;
    if ((rc = alloc((void **)&ws->r, n * 8)) || (rc = alloc((void **)&ws->z, n * 8)) ||
-       (rc = alloc((void **)&ws->t, n * 8)) || (rc = alloc((void **)&ws->partial, (size_t)ws->red_blocks * (m + 2) * 8)) ||
+       (rc = alloc((void **)&ws->t, n * 8)) || (rc = alloc((void **)&ws->partial, (size_t)std::max(ws->red_blocks, ws->gs_blocks) * (m + 2) * 8)) ||
        (rc = alloc((void **)&ws->h, 3 * (size_t)(m + 2) * 8)))
       return rc;
    if ((rc = alloc((void **)&ws->md_count, 16))) return rc;
