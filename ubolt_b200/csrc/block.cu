@@ -6,27 +6,171 @@
 #include "cg.h"
 #include "ctx.h"
 
+#include <algorithm>
+
 namespace ubolt {
 
-template <typename T, int NB, int F, bool TRANS>
-__global__ void BlockApplyKernel(const DevGeom<T> g, const T *__restrict__ x, T *__restrict__ y)
+// What a block solve needs of a class, in shared memory: per face the normal
+// (padded to 4) and face_own, then the gradients and 1 / V, every part on a
+// 16-byte boundary (the class record without face_up)
+template <typename T, int NB, int F>
+struct OwnRecord {
+   static constexpr RecordLayout L = RecordLayout(NB, F, (int)sizeof(T));
+   static constexpr int kUnit = 16 / (int)sizeof(T);
+   static constexpr int kFace = 4 + L.fm, kTail = F * kFace, kSize = kTail + L.size - L.tail;
+   static constexpr int kFaceUnits = kFace / kUnit, kUnits = kSize / kUnit;
+   // Unit u's place in the class record
+   static __device__ __forceinline__ int Source(int u)
+   {
+      constexpr RecordLayout R(NB, F, (int)sizeof(T));
+      const int f = u / kFaceUnits;
+      return f < F ? R.nA(f) + (u - f * kFaceUnits) * kUnit : R.tail + (u - F * kFaceUnits) * kUnit;
+   }
+};
+
+// B r = x solved in place by Gaussian elimination with partial pivoting,
+// without a branch: the largest entry of a column is brought up by
+// conditional row swaps (each row is eliminated by the same arithmetic
+// wherever it stands), and a quotient s / b is s (1 / b) corrected once by its
+// remainder, which rounds as the division does but for the last place. A zero
+// pivot (a singular block) gives zero, as its zeroed inverse does in the reference.
+template <typename T, int NB>
+__device__ __forceinline__ void SolveBlockSelect(T B[NB][NB], T r[NB])
 {
-   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-   if (tid >= g.n_cells * g.A) return;
-   const int64_t c = tid / g.A;
-   const int a = (int)(tid - c * g.A);
-   const T om[3] = {g.omega[3 * a], g.omega[3 * a + 1], g.omega[3 * a + 2]};
-   T B[NB][NB], r[NB];
-   BuildBlock<T, NB, F>(g, g.cls[c], om, g.sigma_t[c], B);
-   if constexpr (TRANS) Transpose<T, NB>(B);
+   T inv[NB];
+   bool singular = false;
 #pragma unroll
-   for (int j = 0; j < NB; j++) r[j] = x[(c * NB + j) * g.A + a];
-   // A singular block maps to zero, as its zeroed inverse does in the reference
-   if (!SolveBlock<T, NB>(B, r))
+   for (int k = 0; k < NB; k++) {
 #pragma unroll
-      for (int j = 0; j < NB; j++) r[j] = T(0);
+      for (int i = k + 1; i < NB; i++) {
+         const bool up = fabs(B[i][k]) > fabs(B[k][k]);
 #pragma unroll
-   for (int j = 0; j < NB; j++) y[(c * NB + j) * g.A + a] = r[j];
+         for (int j = k; j < NB; j++) {
+            const T a = B[k][j], b = B[i][j];
+            B[k][j] = up ? b : a;
+            B[i][j] = up ? a : b;
+         }
+         const T a = r[k], b = r[i];
+         r[k] = up ? b : a;
+         r[i] = up ? a : b;
+      }
+      singular |= B[k][k] == T(0);
+      inv[k] = T(1) / B[k][k];
+#pragma unroll
+      for (int i = k + 1; i < NB; i++) {
+         const T f = B[i][k] * inv[k];
+#pragma unroll
+         for (int j = k + 1; j < NB; j++) B[i][j] -= f * B[k][j];
+         r[i] -= f * r[k];
+      }
+   }
+#pragma unroll
+   for (int k = NB - 1; k >= 0; k--) {
+      T s = r[k];
+#pragma unroll
+      for (int j = k + 1; j < NB; j++) s -= B[k][j] * r[j];
+      const T q = s * inv[k];
+      const T rem = fma(-q, B[k][k], s), better = fma(rem, inv[k], q);
+      r[k] = isfinite(better) ? better : q;  // (an infinite quotient has no remainder)
+   }
+   if (singular)
+#pragma unroll
+      for (int k = 0; k < NB; k++) r[k] = T(0);
+}
+
+constexpr int kBlockThreads = 128;
+// Blocks per SM the registers should leave room for: all that fit without
+// spilling (256^2 triangles, FP64: 97 us at five, 87 at six, 82 at eight; blocks
+// of 256 threads 123)
+template <typename T, int NB>
+constexpr int BlockApplyMinBlocks() { return NB == 1 ? 12 : sizeof(T) == 8 && NB == 4 ? 4 : 8; }
+
+// y = B^{-1} x (or B^{-T} x). A block of 128 threads holds K whole cells, a
+// thread one cell and AP consecutive ordinates at a time (one 16-byte run of
+// each row). The cells' shape data are staged in shared memory by cp.async
+// beside the loads of x. Bound by issue: about 230 instructions per (cell,
+// ordinate), half of them FP64, none behind a branch that splits a warp. A
+// thread per (cell, ordinate) with branches on the signs of the face terms and on
+// the pivots, its shapes gathered through L1, and this kernel, S8, FP64 / FP32:
+// 256^2 triangles 152 / 77 -> 82 / 48 us (0.46 / 0.40 of the copy bandwidth),
+// 301 x 257 quadrilaterals 108 / 50 -> 56 / 35, 48^3 hexahedra 657 / 255 -> 295 /
+// 138, 23 x 21 x 19 cubes of tetrahedra at S6 191 / 75 -> 81 / 47.
+template <typename T, int NB, int F, int AP, bool TRANS>
+__global__ void __launch_bounds__(kBlockThreads, BlockApplyMinBlocks<T, NB>())
+   BlockApplyKernel(const DevGeom<T> g, const T *__restrict__ x, T *__restrict__ y, int K)
+{
+   using Rec = OwnRecord<T, NB, F>;
+   constexpr RecordLayout L(NB, F, (int)sizeof(T));
+   constexpr int kFm = L.fm, kRecSize = L.size;
+   extern __shared__ __align__(16) unsigned char smem_raw[];
+   T *recs = reinterpret_cast<T *>(smem_raw);
+   const int A = g.A, QA = A / AP;
+   const int64_t c0 = (int64_t)blockIdx.x * K;
+   const int kc = (int)min((int64_t)K, g.n_cells - c0);
+   for (int e = threadIdx.x; e < kc * Rec::kUnits; e += kBlockThreads) {
+      const int k = e / Rec::kUnits, u = e - k * Rec::kUnits;
+      CpAsync<16>(recs + k * Rec::kSize + u * Rec::kUnit, g.rec + (int64_t)g.cls[c0 + k] * kRecSize + Rec::Source(u));
+   }
+   bool staged = false;
+   for (int e0 = 0; e0 < kc * QA; e0 += kBlockThreads) {
+      const int e = min(e0 + (int)threadIdx.x, kc * QA - 1);
+      const int k = e / QA, a0 = (e - k * QA) * AP;
+      const int64_t c = c0 + k;
+      T v[NB][AP], om[3 * AP];
+#pragma unroll
+      for (int j = 0; j < NB; j++) LoadRun<T, AP>(x + (c * NB + j) * A + a0, v[j]);
+      LoadRun<T, 3 * AP>(g.omega + 3 * a0, om);
+      const T sigma = g.sigma_t[c];
+      if (!staged) {
+         CpAsyncWaitAll();
+         __syncthreads();
+         staged = true;
+      }
+      const T *rec = recs + k * Rec::kSize;
+#pragma unroll
+      for (int p = 0; p < AP; p++) {
+         // One ordinate after the other: with the matrices read once for all
+         // of them they are kept in registers, and spill
+         asm volatile("" ::: "memory");
+         const T o[3] = {om[3 * p], om[3 * p + 1], om[3 * p + 2]};
+         T B[NB][NB], r[NB];
+#pragma unroll
+         for (int i = 0; i < NB; i++) {
+            r[i] = v[i][p];
+#pragma unroll
+            for (int j = 0; j < NB; j++) B[i][j] = T(0);
+         }
+         if constexpr (NB == 1) {
+            T out = T(0);
+#pragma unroll
+            for (int f = 0; f < F; f++) out += fmax(Dot3(o, rec + f * Rec::kFace), T(0));
+            B[0][0] = out * rec[Rec::kTail] + sigma;
+         } else {
+#pragma unroll
+            for (int f = 0; f < F; f++) {
+               T n[4], m[kFm];
+               LoadShared<T, 4>(rec + f * Rec::kFace, n);
+               LoadShared<T, kFm>(rec + f * Rec::kFace + 4, m);
+               const T s = fmax(Dot3(o, n), T(0));
+#pragma unroll
+               for (int i = 0; i < NB; i++)
+#pragma unroll
+                  for (int j = 0; j < NB; j++) B[i][j] += s * m[i * NB + j];
+            }
+#pragma unroll
+            for (int i = 1; i < NB; i++) B[i][0] -= Dot3(o, rec + Rec::kTail + 3 * i);
+#pragma unroll
+            for (int i = 0; i < NB; i++) B[i][i] += sigma;
+            if constexpr (TRANS) Transpose<T, NB>(B);
+         }
+         SolveBlockSelect<T, NB>(B, r);
+#pragma unroll
+         for (int i = 0; i < NB; i++) v[i][p] = r[i];
+      }
+      if (e0 + (int)threadIdx.x < kc * QA)
+#pragma unroll
+         for (int j = 0; j < NB; j++) StoreRun<T, AP>(y + (c * NB + j) * A + a0, v[j]);
+   }
 }
 
 // Singular-block census (ElementBlockInverse::setup's check,
@@ -72,9 +216,17 @@ __global__ void BlockInverseKernel(const DevGeom<T> g, T *__restrict__ inv)
 template <typename T, int NB, int F>
 static int LaunchBlockApply(const DevGeom<T> &g, const T *x, T *y, bool trans, cudaStream_t s)
 {
-   const int64_t n = g.n_cells * g.A;
-   if (trans) BlockApplyKernel<T, NB, F, true><<<(n + 255) / 256, 256, 0, s>>>(g, x, y);
-   else BlockApplyKernel<T, NB, F, false><<<(n + 255) / 256, 256, 0, s>>>(g, x, y);
+   // Ordinates per thread as one 16-byte run where they divide evenly and both
+   // vectors are 16-byte aligned; as many cells as 128 threads hold
+   constexpr int AV = 16 / (int)sizeof(T);
+   const bool vec = g.A % AV == 0 && (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16 == 0;
+   const int QA = g.A / (vec ? AV : 1);
+   const int K = std::max(1, kBlockThreads / QA);
+   const size_t smem = (size_t)K * OwnRecord<T, NB, F>::kSize * sizeof(T);
+   auto kern = vec ? (trans ? BlockApplyKernel<T, NB, F, AV, true> : BlockApplyKernel<T, NB, F, AV, false>)
+                   : (trans ? BlockApplyKernel<T, NB, F, 1, true> : BlockApplyKernel<T, NB, F, 1, false>);
+   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+   kern<<<(g.n_cells + K - 1) / K, kBlockThreads, smem, s>>>(g, x, y, K);
    return CheckLaunch("block_apply");
 }
 

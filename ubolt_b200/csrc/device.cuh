@@ -12,6 +12,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 #include <cuda_runtime.h>
 
 namespace ubolt {
@@ -164,6 +165,61 @@ __device__ __forceinline__ bool MbarWaitBounded(uint64_t *bar, uint32_t parity, 
    for (uint32_t k = 0; k <= limit; k++)
       if (MbarTryWait(bar, parity)) return true;
    return false;
+}
+
+// N consecutive values from an address aligned to 16 bytes (N * sizeof(T)
+// a multiple of 16), to 8 bytes (8), or element-aligned
+template <typename T, int N>
+__device__ __forceinline__ void LoadRun(const T *__restrict__ p, T v[N])
+{
+   constexpr int B = (int)sizeof(T) * N;
+   if constexpr (B % 16 == 0) {
+#pragma unroll
+      for (int u = 0; u < B / 16; u++) {
+         const int4 w = __ldg(reinterpret_cast<const int4 *>(p) + u);
+         memcpy(&v[u * (16 / (int)sizeof(T))], &w, 16);
+      }
+   } else if constexpr (B == 8 && sizeof(T) == 4) {
+      const int2 w = __ldg(reinterpret_cast<const int2 *>(p));
+      memcpy(v, &w, 8);
+   } else {
+#pragma unroll
+      for (int i = 0; i < N; i++) v[i] = __ldg(p + i);
+   }
+}
+
+template <typename T, int N>
+__device__ __forceinline__ void StoreRun(T *__restrict__ p, const T v[N])
+{
+   constexpr int B = (int)sizeof(T) * N;
+   if constexpr (B % 16 == 0) {
+#pragma unroll
+      for (int u = 0; u < B / 16; u++) {
+         int4 w;
+         memcpy(&w, &v[u * (16 / (int)sizeof(T))], 16);
+         __stcs(reinterpret_cast<int4 *>(p) + u, w);
+      }
+   } else {
+#pragma unroll
+      for (int i = 0; i < N; i++) p[i] = v[i];
+   }
+}
+
+// N consecutive values from shared memory, 16-byte aligned when N *
+// sizeof(T) is a multiple of 16
+template <typename T, int N>
+__device__ __forceinline__ void LoadShared(const T *p, T v[N])
+{
+   if constexpr ((int)sizeof(T) * N % 16 == 0) {
+#pragma unroll
+      for (int u = 0; u < (int)sizeof(T) * N / 16; u++) {
+         const int4 w = reinterpret_cast<const int4 *>(p)[u];
+         memcpy(&v[u * (16 / (int)sizeof(T))], &w, 16);
+      }
+   } else {
+#pragma unroll
+      for (int i = 0; i < N; i++) v[i] = p[i];
+   }
 }
 
 template <typename T>
