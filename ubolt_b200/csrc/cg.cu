@@ -86,42 +86,154 @@ __device__ __forceinline__ T BoundaryTerms(const CgDev<T> &d, int64_t i, int a, 
    return out;
 }
 
-// y = (L - S) x (SCATTER) or L x, one thread per row. phi: the scalar flux of x.
-template <typename T, int DIM, int NV, bool SCATTER>
-__global__ void __launch_bounds__(256) CgApplyKernel(const CgDev<T> d, const T *__restrict__ x,
-                                                     const T *__restrict__ phi, T *__restrict__ y)
+constexpr int kCgThreads = 128;
+// Shared memory of one chunk of star entries
+constexpr int kCgChunkBytes = 48 * 1024;
+
+// Blocks per SM the registers should leave room for: as many as fit without
+// spilling (with the compiler free to take more registers, 256^2 quadrilaterals
+// S8 took 142 us)
+template <typename T, int DIM, int AP>
+constexpr int CgMinBlocks() { return DIM == 2 ? (sizeof(T) == 8 ? 5 : 7) : AP == 1 ? 5 : 4; }
+
+// Bytes of one staged star entry: its record, then per column the scalar flux,
+// the cross sections, the columns and the element
+template <typename T, int DIM, int NV>
+__host__ __device__ constexpr int CgEntryBytes()
 {
-   constexpr int P = CgRecordSize(DIM);
-   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-   if (r >= d.n_rows) return;
-   const int64_t i = r / d.A;
-   const int a = (int)(r - i * d.A);
-   T om[DIM];
+   return NV * CgRecordSize(DIM) * (int)sizeof(T) + (NV + 2) * (int)sizeof(T) + (NV + 1) * 4;
+}
+
+// y = (L - S) x (SCATTER) or L x. phi: the scalar flux of x. A block of 128
+// threads holds K whole vertices, a thread one vertex and AP consecutive
+// ordinates (one 16-byte run of x and y). The star entries of the block's
+// vertices are one contiguous range: their records come into shared memory by
+// cp.async, a chunk of at most E entries at a time, and beside them what does
+// not depend on the ordinate (the columns, their scalar flux, the element and
+// its cross sections), so that the walk over a star waits for nothing but x
+// and tau. Bound by FP64 issue: 12 multiply-adds per (element, column,
+// ordinate), 27 us of them alone at 256^2 quadrilaterals S8. A thread per row
+// that walked its star through L1 (two dependent loads per element, every
+// record read by every ordinate) and this kernel, FP64 / FP32 with the scatter:
+// 256^2 quadrilaterals S8 187 / 107 -> 102 / 52 us, 180^2 triangles S8 111 / 58
+// -> 62 / 35, 30^3 hexahedra S8 721 / 377 -> 266 / 152, 28^3 cubes of tetrahedra
+// S6 687 / 292 -> 268 / 155. Staging the same number of entries of every star
+// at a time, for smaller chunks, took 153 us on the quadrilaterals.
+template <typename T, int DIM, int NV, int AP, bool SCATTER>
+__global__ void __launch_bounds__(kCgThreads, CgMinBlocks<T, DIM, AP>()) CgApplyKernel(const CgDev<T> d, const T *__restrict__ x,
+                                                            const T *__restrict__ phi, T *__restrict__ y, int K, int E)
+{
+   constexpr int P = CgRecordSize(DIM), RS = NV * P;
+   extern __shared__ __align__(16) unsigned char smem_raw[];
+   T *rec = reinterpret_cast<T *>(smem_raw);           // [E][NV][P]
+   T *sphi = rec + (size_t)E * RS;                     // [E][NV]
+   T *ssig = sphi + (size_t)E * NV;                    // [E][2]
+   int32_t *scol = reinterpret_cast<int32_t *>(ssig + (size_t)E * 2);  // [E][NV]
+   int32_t *selem = scol + E * NV;                     // [E]
+   const int A = d.A, QA = A / AP;
+   const int64_t v0 = (int64_t)blockIdx.x * K;
+   const int kc = (int)min((int64_t)K, d.n_vertices - v0);
+   const int first = d.star_off[v0], last = d.star_off[v0 + kc];
+   for (int e0 = 0; e0 < kc * QA; e0 += (int)blockDim.x) {
+      const int idx = min(e0 + (int)threadIdx.x, kc * QA - 1);
+      const int k = idx / QA, a0 = (idx - k * QA) * AP;
+      const int64_t i = v0 + k;
+      const int s0 = d.star_off[i], s1 = d.star_off[i + 1];
+      T om[AP][3], oo[AP][DIM == 2 ? 3 : 6];
+      {
+         T o[3 * AP];
+         LoadRun<T, 3 * AP>(d.omega + 3 * a0, o);
 #pragma unroll
-   for (int c = 0; c < DIM; c++) om[c] = d.omega[3 * a + c];
-   T acc = T(0), sacc = T(0);
-   const int s1 = d.star_off[i + 1];
-   for (int s = d.star_off[i]; s < s1; s++) {
-      const int e = d.star_elem[s];
-      const T st = d.sigma_t[e];
-      const T tau = d.tau[(int64_t)e * d.A + a];
-      const T *rec = d.rec + (int64_t)s * NV * P;
-      const int32_t *col = d.cols + (int64_t)s * NV;
-      T srow = T(0);
+         for (int p = 0; p < AP; p++) {
 #pragma unroll
-      for (int j = 0; j < NV; j++) {
-         const T *q = rec + j * P;
-         const T w = q[0] + tau * DotD<T, DIM>(om, q + 1 + DIM);
-         const T coef = DotD<T, DIM>(om, q + 1) + tau * OmegaKOmega<T, DIM>(q + 1 + 2 * DIM, om) + st * w;
-         const int64_t v = col[j];
-         acc += coef * x[v * d.A + a];
-         if constexpr (SCATTER) srow += w * phi[v];
+            for (int c = 0; c < 3; c++) om[p][c] = o[3 * p + c];
+            const T *w = om[p];
+            oo[p][0] = w[0] * w[0];
+            oo[p][1] = w[1] * w[1];
+            if constexpr (DIM == 2) {
+               oo[p][2] = w[0] * w[1];
+            } else {
+               oo[p][2] = w[2] * w[2];
+               oo[p][3] = w[0] * w[1];
+               oo[p][4] = w[0] * w[2];
+               oo[p][5] = w[1] * w[2];
+            }
+         }
       }
-      if constexpr (SCATTER) sacc += d.sigma_s[e] * srow;
+      T acc[AP], sacc[AP];
+#pragma unroll
+      for (int p = 0; p < AP; p++) acc[p] = sacc[p] = T(0);
+      for (int c0 = first; c0 < last; c0 += E) {
+         const int n = min(E, last - c0);
+         // The block holds one chunk; it is staged again only where there are more
+         if (last - first > E || e0 == 0) {
+            __syncthreads();
+            const unsigned char *src = reinterpret_cast<const unsigned char *>(d.rec + (int64_t)c0 * RS);
+            for (int u = threadIdx.x; u < n * (RS * (int)sizeof(T) / 16); u += (int)blockDim.x)
+               CpAsync<16>(smem_raw + 16 * u, src + 16 * u);
+            for (int u = threadIdx.x; u < n * NV; u += (int)blockDim.x) {
+               const int32_t v = d.cols[(int64_t)c0 * NV + u];
+               scol[u] = v;
+               if constexpr (SCATTER) sphi[u] = phi[v];
+            }
+            for (int u = threadIdx.x; u < n; u += (int)blockDim.x) {
+               const int32_t e = d.star_elem[c0 + u];
+               selem[u] = e;
+               ssig[2 * u] = d.sigma_t[e];
+               if constexpr (SCATTER) ssig[2 * u + 1] = d.sigma_s[e];
+            }
+            CpAsyncWaitAll();
+            __syncthreads();
+         }
+         const int lo = max(s0 - c0, 0), hi = min(s1 - c0, n);
+#pragma unroll (DIM == 2 ? 1 : 2)
+         for (int s = lo; s < hi; s++) {
+            T tau[AP], xv[NV][AP], srow[AP];
+            LoadRun<T, AP>(d.tau + (int64_t)selem[s] * A + a0, tau);
+#pragma unroll
+            for (int j = 0; j < NV; j++) LoadRun<T, AP>(x + (int64_t)scol[s * NV + j] * A + a0, xv[j]);
+            const T st = ssig[2 * s];
+#pragma unroll
+            for (int p = 0; p < AP; p++) srow[p] = T(0);
+#pragma unroll
+            for (int j = 0; j < NV; j++) {
+               T q[P];
+               LoadShared<T, P>(rec + (s * NV + j) * P, q);
+#pragma unroll
+               for (int p = 0; p < AP; p++) {
+                  T og = T(0), gt = T(0), kk = T(0);
+#pragma unroll
+                  for (int c = 0; c < DIM; c++) {
+                     og += om[p][c] * q[1 + c];
+                     gt += om[p][c] * q[1 + DIM + c];
+                  }
+#pragma unroll
+                  for (int c = 0; c < (DIM == 2 ? 3 : 6); c++) kk += oo[p][c] * q[1 + 2 * DIM + c];
+                  const T w = q[0] + tau[p] * gt;
+                  acc[p] += (og + tau[p] * kk + st * w) * xv[j][p];
+                  if constexpr (SCATTER) srow[p] += w * sphi[s * NV + j];
+               }
+            }
+            if constexpr (SCATTER)
+#pragma unroll
+               for (int p = 0; p < AP; p++) sacc[p] += ssig[2 * s + 1] * srow[p];
+         }
+      }
+      if (e0 + (int)threadIdx.x < kc * QA) {
+         const T im = d.inv_m[i];
+         T out[AP];
+#pragma unroll
+         for (int p = 0; p < AP; p++) {
+            T v = acc[p];
+            if constexpr (SCATTER) v -= sacc[p] * d.inv_sum_weights;
+            T o[DIM];
+#pragma unroll
+            for (int c = 0; c < DIM; c++) o[c] = om[p][c];
+            out[p] = v * im + BoundaryTerms<T, DIM>(d, i, a0 + p, o, x);
+         }
+         StoreRun<T, AP>(y + i * A + a0, out);
+      }
    }
-   T out = acc;
-   if constexpr (SCATTER) out -= sacc * d.inv_sum_weights;
-   y[r] = out * d.inv_m[i] + BoundaryTerms<T, DIM>(d, i, a, om, x);
 }
 
 // The diagonal of L (the assembled term's diagonal slot, SUPGTermCG::
@@ -289,6 +401,29 @@ static int EnsureTau(ubolt_ctx *ctx, cudaStream_t s)
    return rc;
 }
 
+template <typename T, int DIM, int NV>
+static int LaunchCgApply(const CgDev<T> &d, int max_star, const T *x, const T *phi, T *y, bool scatter, cudaStream_t s)
+{
+   // As many vertices per block as 128 threads hold and as their star entries
+   // fit in one chunk (few ordinates on hexahedra: 8 entries of 1 KB a vertex).
+   // Ordinates per thread as one 16-byte run where they divide evenly and both
+   // vectors are 16-byte aligned, unless that leaves a block few threads
+   // (20^3 hexahedra S2, FP64: 74 us with runs in chunks against 43)
+   constexpr int AV = 16 / (int)sizeof(T);
+   constexpr int kEntry = CgEntryBytes<T, DIM, NV>(), kMost = kCgChunkBytes / kEntry;
+   const int fit = std::max(1, kMost / max_star);
+   const bool aligned = d.A % AV == 0 && (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16 == 0;
+   const bool vec = aligned && (int64_t)fit * (d.A / AV) >= kCgThreads / 2;
+   const int QA = d.A / (vec ? AV : 1);
+   const int K = std::max(1, std::min(fit, kCgThreads / QA));
+   const int E = std::min(K * max_star, kMost);
+   const int threads = std::min(kCgThreads, (K * QA + 31) / 32 * 32);
+   auto kern = vec ? (scatter ? CgApplyKernel<T, DIM, NV, AV, true> : CgApplyKernel<T, DIM, NV, AV, false>)
+                   : (scatter ? CgApplyKernel<T, DIM, NV, 1, true> : CgApplyKernel<T, DIM, NV, 1, false>);
+   kern<<<(unsigned)((d.n_vertices + K - 1) / K), threads, (size_t)E * kEntry, s>>>(d, x, phi, y, K, E);
+   return CheckLaunch("cg apply");
+}
+
 template <typename T>
 int CgApply(ubolt_ctx *ctx, const T *x, T *y, bool scatter, void *stream)
 {
@@ -308,11 +443,8 @@ int CgApply(ubolt_ctx *ctx, const T *x, T *y, bool scatter, void *stream)
       }
       if (rc) return rc;
    }
-   UBOLT_CG_DISPATCH(cg->dim, cg->nv, {
-      if (scatter) CgApplyKernel<T, D_, N_, true><<<Grid(d.n_rows), 256, 0, s>>>(d, x, phi, y);
-      else CgApplyKernel<T, D_, N_, false><<<Grid(d.n_rows), 256, 0, s>>>(d, x, phi, y);
-   });
-   return CheckLaunch("cg apply");
+   UBOLT_CG_DISPATCH(cg->dim, cg->nv, return (LaunchCgApply<T, D_, N_>(d, cg->max_star, x, phi, y, scatter, s)));
+   return SetError(UBOLT_ERR_STATE, "no CG-SUPG kernel for this shape");
 }
 template int CgApply<double>(ubolt_ctx *, const double *, double *, bool, void *);
 template int CgApply<float>(ubolt_ctx *, const float *, float *, bool, void *);
@@ -479,6 +611,8 @@ extern "C" int ubolt_ctx_create_cg(const ubolt_cg_geometry *geom, const ubolt_qu
    cg->n_vertices = nvx;
    cg->n_elements = ne;
    cg->n_star = ns;
+   for (int64_t v = 0; v < nvx; v++)
+      cg->max_star = std::max<int>(cg->max_star, (int)(geom->star_offset[v + 1] - geom->star_offset[v]));
    cg->zeta = zeta;
 
    // ~~~~~ Sides: one family each, from the boundary faces

@@ -41,6 +41,7 @@ struct CgDev {
 struct ubolt_cg {
    int dim = 0, nv = 0, F = 0, P = 0;
    int64_t n_vertices = 0, n_elements = 0, n_star = 0;
+   int max_star = 1;  // most elements around a vertex
    double zeta = 0.5;
    ubolt::CgDev<double> d64{};
    ubolt::CgDev<float> d32{};
