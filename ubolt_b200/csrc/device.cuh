@@ -449,51 +449,123 @@ __host__ inline int CellsPerBlock(int A)
    return k < 1 ? 1 : k;
 }
 
-// The factors of one (cell, ordinate) for the sweep: W = B^{-1} of its
-// streaming + removal block, and G_s = W (s_f face_up_f) for each gathered
-// face f in face order (slot s); element (s, ii, j) goes to Gout[s * gs + ii * gr + j * gj].
-// A singular block gives zero factors. Returns false then.
-template <typename T, int NB, int F>
-__device__ __forceinline__ bool CellFactors(const DevGeom<T> &g, int64_t c, const T om[3], uint32_t mask, T W[NB][NB],
+// The explicit inverse as InvertBlock's, without a branch: the largest entry of
+// a column comes up by conditional row swaps, which leave every row's
+// arithmetic as it is. False on a zero pivot, with w not to be used.
+template <typename T, int NB>
+__device__ __forceinline__ bool InvertBlockSelect(T m[NB][NB], T w[NB][NB])
+{
+   bool ok = true;
+#pragma unroll
+   for (int i = 0; i < NB; i++)
+#pragma unroll
+      for (int j = 0; j < NB; j++) w[i][j] = (i == j) ? T(1) : T(0);
+#pragma unroll
+   for (int k = 0; k < NB; k++) {
+#pragma unroll
+      for (int i = k + 1; i < NB; i++) {
+         const bool up = fabs(m[i][k]) > fabs(m[k][k]);
+#pragma unroll
+         for (int j = 0; j < NB; j++) {
+            const T a = m[k][j], b = m[i][j], c = w[k][j], e = w[i][j];
+            m[k][j] = up ? b : a;
+            m[i][j] = up ? a : b;
+            w[k][j] = up ? e : c;
+            w[i][j] = up ? c : e;
+         }
+      }
+      ok &= m[k][k] != T(0);
+      const T inv_piv = T(1) / m[k][k];
+#pragma unroll
+      for (int j = 0; j < NB; j++) { m[k][j] *= inv_piv; w[k][j] *= inv_piv; }
+#pragma unroll
+      for (int i = 0; i < NB; i++) {
+         if (i == k) continue;
+         const T f = m[i][k];
+#pragma unroll
+         for (int j = 0; j < NB; j++) { m[i][j] -= f * m[k][j]; w[i][j] -= f * w[k][j]; }
+      }
+   }
+   return ok;
+}
+
+// The factors of one (cell, ordinate) for the sweep, from the cell's class
+// record (in shared or global memory): W = B^{-1} of its streaming + removal
+// block, and G_s = W (s_f face_up_f) for each gathered face f of `mask` in face
+// order (slot s < S; unused slots zero); element (s, ii, j) goes to
+// Gout[s * gs + ii * gr + j * gj]. A singular block gives zero factors. With
+// the records in shared memory (SHARED) no lane branches on its own; from
+// global memory, where the lanes' cells lie on lines of their own and the
+// loads are what costs, a face's matrix is read only where it counts.
+template <typename T, int NB, int F, bool SHARED>
+__device__ __forceinline__ void CellFactors(const T *rec, T sigma_t, const T om[3], uint32_t mask, int S, T W[NB][NB],
                                             T *Gout, size_t gs, size_t gr, size_t gj)
 {
-   const int32_t cl = g.cls[c];
-   T B[NB][NB];
-   BuildBlock<T, NB, F>(g, cl, om, g.sigma_t[c], B);
-   const bool ok = InvertBlock<T, NB>(B, W);
-   if (!ok)
+   constexpr RecordLayout L(NB, F, (int)sizeof(T));
+   constexpr int kFm = L.fm > 0 ? L.fm : 1, kTail = L.size - L.tail;
+   T B[NB][NB], tail[kTail];
+   LoadShared<T, kTail>(rec + L.tail, tail);
 #pragma unroll
-      for (int ii = 0; ii < NB; ii++)
+   for (int i = 0; i < NB; i++)
 #pragma unroll
-         for (int j = 0; j < NB; j++) W[ii][j] = T(0);
-   int slot = 0;
+      for (int j = 0; j < NB; j++) B[i][j] = T(0);
 #pragma unroll
    for (int f = 0; f < F; f++) {
-      if (!(((mask >> f) | (mask >> (8 + f))) & 1u)) continue;
-      const T sf = Dot3(om, g.nA + ((int64_t)cl * F + f) * 3);
+      T n[4];
+      LoadShared<T, 4>(rec + L.nA(f), n);
+      const T s = fmax(Dot3(om, n), T(0));
+      if constexpr (NB == 1) {
+         B[0][0] += s;
+      } else if (SHARED || s > T(0)) {
+         T m[kFm];
+         LoadShared<T, kFm>(rec + L.fown(f), m);
+#pragma unroll
+         for (int i = 0; i < NB; i++)
+#pragma unroll
+            for (int j = 0; j < NB; j++) B[i][j] += s * m[i * NB + j];
+      }
+   }
+   if constexpr (NB == 1) {
+      B[0][0] = B[0][0] * tail[0] + sigma_t;
+   } else {
+#pragma unroll
+      for (int i = 1; i < NB; i++) B[i][0] -= Dot3(om, tail + 3 * i);
+#pragma unroll
+      for (int i = 0; i < NB; i++) B[i][i] += sigma_t;
+   }
+   const bool ok = InvertBlockSelect<T, NB>(B, W);
+#pragma unroll
+   for (int ii = 0; ii < NB; ii++)
+#pragma unroll
+      for (int j = 0; j < NB; j++) W[ii][j] = ok ? W[ii][j] : T(0);
+   uint32_t left = (mask | (mask >> 8)) & 0xffu;
+#pragma unroll 1
+   for (int slot = 0; slot < S; slot++) {
+      const bool used = left != 0;
+      const int f = used ? __ffs(left) - 1 : 0;
+      left &= left - 1;
+      T n[4];
+      LoadShared<T, 4>(rec + L.nA(f), n);
+      const T sf = used ? Dot3(om, n) : T(0);
       T *Gf = Gout + (size_t)slot * gs;
       if constexpr (NB == 1) {
-         Gf[0] = W[0][0] * (sf * g.inv_vol[cl]);
+         Gf[0] = used ? W[0][0] * (sf * tail[0]) : T(0);
       } else {
-         const T *M = g.fup + ((int64_t)cl * F + f) * NB * NB;
-         T Ms[NB][NB];
+         T m[kFm];
+         LoadShared<T, kFm>(rec + L.fup(f), m);
 #pragma unroll
-         for (int kk = 0; kk < NB; kk++)
-#pragma unroll
-            for (int j = 0; j < NB; j++) Ms[kk][j] = sf * M[kk * NB + j];
+         for (int k = 0; k < NB * NB; k++) m[k] = used ? sf * m[k] : T(0);
 #pragma unroll
          for (int ii = 0; ii < NB; ii++)
 #pragma unroll
             for (int j = 0; j < NB; j++) {
                T u = T(0);
 #pragma unroll
-               for (int kk = 0; kk < NB; kk++) u += W[ii][kk] * Ms[kk][j];
+               for (int kk = 0; kk < NB; kk++) u += W[ii][kk] * m[kk * NB + j];
                Gf[(size_t)ii * gr + (size_t)j * gj] = u;
             }
       }
-      slot++;
    }
-   return ok;
 }
 
 // A grid barrier's arrival and wait, by one thread of a block of a cooperative

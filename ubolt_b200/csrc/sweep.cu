@@ -99,6 +99,8 @@ struct ubolt_sweep_plan {
    const uint16_t *tmask = nullptr;     // upwind faces: in task (bit f) / earlier task (bit 8 + f)
    const uint16_t *pass = nullptr;      // end positions of every task's passes (levels cut at 32 / nb positions)
    const int32_t *ghost = nullptr;      // the cells of earlier tasks each task reads
+   const int32_t *patch_ptr = nullptr;  // [n_patches + 1] each patch's tasks in patch_task
+   const int32_t *patch_task = nullptr; // [n_tasks]
    int n_loc = 0;                       // most (positions + ghosts) of a task, plus one
    int n_ghost = 1;                     // most ghosts of a task
    uint32_t *ctrl = nullptr;            // [kCtrlCounter] task counter; [kCtrlError] error flag, [kCtrlError + 1] timeout count
@@ -315,6 +317,9 @@ struct SweepDev {
 // unit is added there
 __host__ __device__ constexpr int LaneStride(int gc, int elem) { return gc * elem % 64 == 0 ? gc + 16 / elem : gc; }
 
+// The stride between staged class records, odd in 16-byte units
+__host__ __device__ constexpr int RecordStride(int size, int elem) { return (size * elem / 16 | 1) * 16 / elem; }
+
 struct SweepSlice {
    int loc, G, rec, pass, ghost, bar, bytes;
    __host__ __device__ constexpr SweepSlice(int P, int S, int F, int NB, int n_loc, int n_ghost, int elem, bool cached)
@@ -339,55 +344,67 @@ struct SweepSlice {
 // lane of the walk reads is one run. Unused slots are zero. Independent of the
 // right-hand side: built once per group, read by every sweep. The couplings
 // are laid out in shared memory and written 32 positions at a time.
-// Slots from..S of a position's couplings set to zero
-template <typename T, int NB>
-__device__ __forceinline__ void ZeroSlots(T *G, int from, int S)
+// A block takes a patch: its cells' class records are staged in shared memory
+// once (STAGED, where they fit) and read by the tasks of every ordinate, a warp
+// per task. Read by a lane per position straight from global memory, every
+// load touched 32 lines, which bound the kernel (and the factors built in the
+// sweep itself). A group's factors, FP64 / FP32, a warp per task from global
+// memory and this way: 256^2 triangles S8 733 / 424 -> 448 / 300 us, 20^3 cubes
+// of tetrahedra 2095 / 1348 -> 1044 / 555, 40^3 hexahedra 2272 / 2041 -> 969 /
+// 477; a few hundred thousand cell-ordinates, where a patch's blocks are few,
+// 59 / 37 -> 75 / 41 (101 x 77 triangles S6).
+template <typename T, int NB, int F, bool STAGED>
+__global__ void __launch_bounds__(256, sizeof(T) == 8 && NB == 4 ? 1 : 2) FactorKernel(const DevGeom<T> g, const SweepDev s, T *__restrict__ fac,
+                                                    const int32_t *__restrict__ patch_ptr,
+                                                    const int32_t *__restrict__ patch_task)
 {
-   for (int sl = from; sl < S; sl++)
-#pragma unroll
-      for (int e = 0; e < NB * NB; e++) G[(e / NB) * S * NB + sl * NB + e % NB] = T(0);
-}
-
-template <typename T, int NB, int F>
-__global__ void __launch_bounds__(128) FactorKernel(const DevGeom<T> g, const SweepDev s, T *__restrict__ fac)
-{
+   constexpr int RS = RecordLayout(NB, F, (int)sizeof(T)).size;
+   constexpr int RP = RecordStride(RS, (int)sizeof(T));
    extern __shared__ __align__(16) unsigned char smem_raw[];
-   const int lane = threadIdx.x & 31;
-   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
    const int S = s.slots, GC = S * NB * NB;
    const int GP = LaneStride(GC, (int)sizeof(T));
-   T *stage = reinterpret_cast<T *>(smem_raw) + (size_t)(threadIdx.x >> 5) * 32 * GP;
+   T *recs = reinterpret_cast<T *>(smem_raw);
+   T *stage = recs + (STAGED ? (size_t)s.P * RP : 0) + (size_t)warp * 32 * GP;
    const unsigned magic = ((1u << 20) + GC - 1) / GC;  // e / GC for e < 32 GC, GC <= 80 (exact: e * GC < 2^20)
    const size_t R = (size_t)NB * NB * (1 + S);
-   for (int64_t t = warp; t < s.n_tasks; t += n_warps) {
-      const Task tk = LoadTask(s.task + t);
-      const int ncell = tk.ncell();
-      const int a = tk.ordinate;
-      const int64_t base = (int64_t)tk.patch * s.P;
+   const int64_t base = (int64_t)blockIdx.x * s.P;
+   if constexpr (STAGED) {
+      constexpr int UN = RS * (int)sizeof(T) / 16;
+      const int nc = (int)min((int64_t)s.P, g.n_cells - base);
+      for (int e = threadIdx.x; e < nc * UN; e += blockDim.x) {
+         const int k = e / UN, u = e - k * UN;
+         CpAsync<16>(recs + k * RP + u * (16 / (int)sizeof(T)),
+                     g.rec + (int64_t)g.cls[base + k] * RS + u * (16 / (int)sizeof(T)));
+      }
+      CpAsyncWaitAll();
+      __syncthreads();
+   }
+   for (int32_t x = patch_ptr[blockIdx.x] + warp + n_warps * (int)blockIdx.y; x < patch_ptr[blockIdx.x + 1];
+        x += n_warps * (int)gridDim.y) {
+      const Task tk = LoadTask(s.task + patch_task[x]);
+      const int ncell = tk.ncell(), a = tk.ordinate;
       const T om[3] = {g.omega[3 * a], g.omega[3 * a + 1], g.omega[3 * a + 2]};
       T *ft = fac + (size_t)tk.off * R;
       for (int i0 = 0; i0 < ncell; i0 += 32) {
-         const int i = i0 + lane;
-         if (i < ncell) {
-            T W[NB][NB];
-            const uint32_t mask = s.tmask[tk.off + i];
-            T *Gi = stage + lane * GP;
-            CellFactors<T, NB, F>(g, base + s.sched[(tk.off + i) * SchedWords(F)], om, mask, W, Gi, (size_t)NB,
-                                  (size_t)S * NB, 1);
-            ZeroSlots<T, NB>(Gi, __popc((mask | (mask >> 8)) & 0xffu), S);
+         // A lane past the end repeats the last position
+         const int i = min(i0 + lane, ncell - 1);
+         const int local = s.sched[(tk.off + i) * SchedWords(F)];
+         const T *rec = STAGED ? recs + local * RP : g.rec + (int64_t)g.cls[base + local] * RS;
+         T W[NB][NB];
+         CellFactors<T, NB, F, STAGED>(rec, g.sigma_t[base + local], om, s.tmask[tk.off + i], S, W, stage + lane * GP, (size_t)NB,
+                               (size_t)S * NB, 1);
 #pragma unroll
-            for (int ii = 0; ii < NB; ii++)
+         for (int ii = 0; ii < NB; ii++)
 #pragma unroll
-               for (int j = 0; j < NB; j++) ft[(size_t)(ii * NB + j) * ncell + i] = W[ii][j];
-         }
+            for (int j = 0; j < NB; j++) ft[(size_t)(ii * NB + j) * ncell + i] = W[ii][j];
          __syncwarp();
          T *Gt = ft + (size_t)NB * NB * ncell + (size_t)i0 * GC;
          const int n = min(32, ncell - i0) * GC;
 #pragma unroll 4
          for (int e = lane; e < n; e += 32) {
-            const int i = (int)((e * magic) >> 20);
-            Gt[e] = stage[i * GP + (e - i * GC)];
+            const int q = (int)((e * magic) >> 20);
+            Gt[e] = stage[q * GP + (e - q * GC)];
          }
          __syncwarp();
       }
@@ -543,10 +560,9 @@ __global__ void __launch_bounds__(64, SweepMinBlocks<T, NB, S, KU>()) SweepKerne
                if (i0 + 32 * k + lane >= ncell) continue;
                const T om[3] = {g.omega[3 * a], g.omega[3 * a + 1], g.omega[3 * a + 2]};
                T *Gi = G + i * GP;
-               const uint32_t mask = s.tmask[off + i];
-               CellFactors<T, NB, F>(g, base + (int)(rec[k].x & 0xffffu), om, mask, W[k], Gi, (size_t)NB,
-                                     (size_t)S * NB, 1);
-               ZeroSlots<T, NB>(Gi, __popc((mask | (mask >> 8)) & 0xffu), S);
+               const int64_t c = base + (int)(rec[k].x & 0xffffu);
+               CellFactors<T, NB, F, false>(g.rec + (int64_t)g.cls[c] * RecordLayout(NB, F, EL).size, g.sigma_t[c], om,
+                                     s.tmask[off + i], S, W[k], Gi, (size_t)NB, (size_t)S * NB, 1);
             }
 #pragma unroll
             for (int ii = 0; ii < NB; ii++) {
@@ -892,8 +908,16 @@ int BuildSweepPlan(ubolt_ctx *ctx, int patch_size)
          task[t].ghost0 += ghost_at[k];
       }
    }
+   std::vector<int32_t> patch_ptr(h.n_patches + 1, 0), patch_task(h.n_tasks);
+   for (int64_t t = 0; t < h.n_tasks; t++) patch_ptr[task[t].patch + 1]++;
+   for (int32_t k = 0; k < h.n_patches; k++) patch_ptr[k + 1] += patch_ptr[k];
+   {
+      std::vector<int32_t> at(patch_ptr.begin(), patch_ptr.end() - 1);
+      for (int64_t t = 0; t < h.n_tasks; t++) patch_task[at[task[t].patch]++] = (int32_t)t;
+   }
    int rc = 0;
-   if ((rc = UploadVec(ctx, task, &plan->task)) || (rc = UploadVec(ctx, h.dep_ptr, &plan->dep_ptr)) ||
+   if ((rc = UploadVec(ctx, patch_ptr, &plan->patch_ptr)) || (rc = UploadVec(ctx, patch_task, &plan->patch_task)) ||
+       (rc = UploadVec(ctx, task, &plan->task)) || (rc = UploadVec(ctx, h.dep_ptr, &plan->dep_ptr)) ||
        (rc = UploadVec(ctx, h.deps, &plan->deps)) || (rc = UploadVec(ctx, sched, &plan->sched)) ||
        (rc = UploadVec(ctx, h.tmask, &plan->tmask)) || (rc = UploadVec(ctx, pass, &plan->pass)) ||
        (rc = UploadVec(ctx, ghost, &plan->ghost))) {
@@ -1088,13 +1112,22 @@ static T *EnsureFactors(ubolt_ctx *ctx, cudaStream_t st)
       pl->fac_epoch[which] = ctx->group_epoch;
       return static_cast<T *>(pl->fac[which]);
    }
-   int n_sm = 0, dev = 0;
+   int smem_max = 48 * 1024, dev = 0;
    cudaGetDevice(&dev);
-   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-   const int64_t grid = std::min<int64_t>((pl->n_tasks + 3) / 4, (int64_t)n_sm * 16);
-   const int smem = 4 * 32 * LaneStride(pl->slots * NB * NB, (int)sizeof(T)) * (int)sizeof(T);
-   if (smem > 48 * 1024) cudaFuncSetAttribute(FactorKernel<T, NB, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-   FactorKernel<T, NB, F><<<(int)grid, 128, smem, st>>>(ctx->geom<T>(), DevPlan(pl), static_cast<T *>(pl->fac[which]));
+   cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+   // Eight warps per patch, four where the patches are few; its class
+   // records in shared memory where they fit beside the warps' staging
+   const int warps = 8;
+   const size_t stage = (size_t)warps * 32 * LaneStride(pl->slots * NB * NB, (int)sizeof(T)) * sizeof(T);
+   const size_t recs = (size_t)pl->P * RecordStride(RecordLayout(NB, F, (int)sizeof(T)).size, (int)sizeof(T)) * sizeof(T);
+   const bool staged = recs + stage <= (size_t)smem_max;
+   const size_t smem = (staged ? recs : 0) + stage;
+   auto kern = staged ? FactorKernel<T, NB, F, true> : FactorKernel<T, NB, F, false>;
+   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+   // Large patches make few blocks: then several share a patch's tasks
+   const int parts = std::max(1, std::min((148 * 8 + pl->n_patches - 1) / pl->n_patches, (ctx->A + warps - 1) / warps));
+   kern<<<dim3(pl->n_patches, parts), 32 * warps, smem, st>>>(ctx->geom<T>(), DevPlan(pl), static_cast<T *>(pl->fac[which]),
+                                                 pl->patch_ptr, pl->patch_task);
    if (CheckLaunch("sweep factors")) return nullptr;
    pl->fac_epoch[which] = ctx->group_epoch;
    return static_cast<T *>(pl->fac[which]);

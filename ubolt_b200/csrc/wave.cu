@@ -59,7 +59,8 @@ __global__ void __launch_bounds__(128) WaveFactorKernel(const DevGeom<T> g, cons
          const int4 m = w.meta[(int64_t)a * w.n_cells + p0 + i];
          const uint32_t mask = ((uint32_t)m.y >> 16) & 0xffu;
          T W[NB][NB];
-         CellFactors<T, NB, F>(g, m.x, om, mask, W, ck + (size_t)NB * NB * n + i, (size_t)NB * NB * n,
+         const T *rec = g.rec + (int64_t)g.cls[m.x] * RecordLayout(NB, F, (int)sizeof(T)).size;
+         CellFactors<T, NB, F, false>(rec, g.sigma_t[m.x], om, mask, w.S, W, ck + (size_t)NB * NB * n + i, (size_t)NB * NB * n,
                                (size_t)NB * n, (size_t)n);
 #pragma unroll
          for (int ii = 0; ii < NB; ii++)
