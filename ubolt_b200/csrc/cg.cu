@@ -10,11 +10,11 @@
 //              - 1/m_i sum_e sigma_s / W sum_j (M_ij + tau Omega.G_ji) phi(j)
 //   tau(e, a) = min(1 / sigma_t, 2 / (zeta sum_j |Omega_a . grad phi_j(x_c)|)).
 // The reference assembles the first two lines into a matrix per group and
-// applies the scatter matrix-free; here one thread per row gathers all three
-// from the element tables, so there is no matrix to refill per group.
-// A row's (element, column) coefficients are needed by the A threads of its
-// vertex at once: the star records are laid out vertex-major, so those
-// threads read the same addresses (one L1 line serves the warp).
+// applies the scatter matrix-free; here all three are gathered from the
+// element tables, so there is no matrix to refill per group.
+// A row's (element, column) coefficients are needed by every ordinate of its
+// vertex: the star records are laid out vertex-major, and the multiply stages
+// them in shared memory once for all of its vertices' ordinates.
 #include "cg.h"
 
 #include <algorithm>
