@@ -88,6 +88,17 @@ __host__ __device__ constexpr size_t ApplySmemElems(int K, int threads, int A, b
 template <typename T, int NB, int AP>
 constexpr int ApplyMinBlocks() { return (NB == 4 && AP > 1) ? 2 : 3; }
 
+// True where the grid is one wave of resident blocks that walk the cells in
+// rounds, keeping their ordinates and weights: the two-block-per-SM kernels of
+// DG1 tets and hexes, where a block's start is a larger share. Measured, a
+// block per group of cells and rounds: 64^3 hexes S8 FP32 470 and 434 us,
+// 23 x 21 x 19 cubes of tets S6 FP64 transposed 117.5 and 107 (454 and 111 with
+// the codes and class read where the copies need them, not at a round's start); 256^2 triangles
+// FP64, with three blocks at the 80-register cap, 134 and 138 (the loop's state
+// spills), which stay a block per group
+template <int NB, int F, int AP>
+constexpr bool ApplyRounds() { return UpSlots<NB, F>() < F && AP > 1; }
+
 // REV: the transpose (L - S)^T = L^T - S^T, L^T as the reversed-angle
 // operator. (V L)^T = P (V L) P (V the cell volume on every row, P the swap
 // of each ordinate with its opposite) gives L^T x = P V L (P V^{-1} x): the
@@ -106,6 +117,7 @@ __global__ void __launch_bounds__(256, ApplyMinBlocks<T, NB, AP>()) ApplyKernel(
    constexpr int RU = L.size * (int)sizeof(T) / 16;
    constexpr int XS = UpSlots<NB, F>();
    constexpr bool kRing = XS < F;
+   constexpr bool kRounds = ApplyRounds<NB, F, AP>();
    extern __shared__ __align__(16) unsigned char smem_raw[];
    const int A = g.A, QA = A / AP;
    T *recs = reinterpret_cast<T *>(smem_raw);
@@ -122,218 +134,237 @@ __global__ void __launch_bounds__(256, ApplyMinBlocks<T, NB, AP>()) ApplyKernel(
    // The run of x read for this cell and its neighbours, and of y written:
    // this thread's ordinates, or (REV) their opposites, the same run reversed
    const int ar0 = REV ? g.opp[a0 + AP - 1] : a0;
-   const int64_t c0 = (int64_t)blockIdx.x * K;
-   const int64_t c = c0 + k;
-   const int kc = (int)min((int64_t)K, g.n_cells - c0);
-   const bool live = k < kc;
-
-   // Stage: the block's own rows (one contiguous range), each cell's class
-   // record and this thread's upwind runs, all in flight at once (with the
-   // ring, the first two faces' runs, each in a commit group of its own).
-   // Per face 4 bits of fcode: 8 for an interior face, else the boundary side.
-   unsigned fcode = 0;
-   {
-      const int nu = kc * NB * A * (int)sizeof(T) / CU;
-      const unsigned char *src = reinterpret_cast<const unsigned char *>(x + c0 * NB * A);
-      for (int u = t; u < nu; u += blockDim.x) CpAsyncRun<CU>(reinterpret_cast<unsigned char *>(xs) + u * CU, src + u * CU);
-   }
-   if (live) {
-      const T *rec = g.rec + (int64_t)g.cls[c] * L.size;
-      for (int u = q; u < RU; u += QA) CpAsync<16>(recs + k * L.size + u * (16 / (int)sizeof(T)), rec + u * (16 / (int)sizeof(T)));
-      if constexpr (kRing) CpAsyncCommit();
-      T vc = T(0);
-      if constexpr (REV) vc = g.volume[c];
-#pragma unroll
-      for (int f = 0; f < F; f++) {
-         const int32_t cf = g.code[c * F + f];
-         if (FaceInterior(cf)) {
-            fcode |= 8u << (4 * f);
-            if constexpr (REV) rat[f * (int)blockDim.x + t] = vc * g.inv_vol[g.cls[cf]];
-            if (!kRing || f < XS) {
-#pragma unroll
-               for (int j = 0; j < NB; j++)
-                  CpAsyncRun<CU>(xup + ((f * NB + j) * (int)blockDim.x + t) * AP, x + ((int64_t)cf * NB + j) * A + ar0);
-            }
-         } else {
-            fcode |= (unsigned)FaceSide(cf) << (4 * f);
-         }
-         if (kRing && f < XS) CpAsyncCommit();
-      }
-   }
    T om[3 * AP];
-   T sig_t = T(0);
-   if (live) {
-      LoadRun<T, 3 * AP>(g.omega + 3 * a0, om);
-      sig_t = g.sigma_t[c];
-      if (SCATTER && q == 0) ssw[k] = g.sigma_s[c] * g.inv_sum_weights;
+   if constexpr (kRounds) {
+      if (k < K) LoadRun<T, 3 * AP>(g.omega + 3 * a0, om);
+      if constexpr (SCATTER)
+         for (int b = t; b < A; b += blockDim.x) ws[b] = g.w[b];
    }
-   if constexpr (SCATTER)
-      for (int b = t; b < A; b += blockDim.x) ws[b] = g.w[b];
-   // The shared rows and records are in; with the ring, a live thread's two
-   // face groups may still be in flight (a thread without a cell committed
-   // no group, so it waits for all of its copies)
-   if (kRing && live) CpAsyncWaitGroup<XS>();
-   else CpAsyncWaitAll();
-   __syncthreads();
+   for (int64_t c0 = (int64_t)blockIdx.x * K; !kRounds || c0 < g.n_cells; c0 += (int64_t)gridDim.x * K) {
+      const int64_t c = c0 + k;
+      const int kc = (int)min((int64_t)K, g.n_cells - c0);
+      const bool live = k < kc;
+      int32_t code[F], cls = 0;
+      // Read together, before any copy: the copies are ordered among themselves,
+      // so a code read between two of them would wait alone (256^2 triangles FP64
+      // 134 -> 131 us)
+      if (live) {
+         cls = g.cls[c];
+#pragma unroll
+         for (int f = 0; f < F; f++) code[f] = g.code[c * F + f];
+      }
 
-   if constexpr (SCATTER) {
-      // sigma_s / W sum_b w_b x(node, b) from the staged rows: four lanes
-      // per node, each a fixed quarter of the ordinates, then two shuffles.
-      // The loop bound is the same for every thread (the shuffles need the
-      // whole warp).
-      constexpr int G = 4;
-      const int nodes = kc * NB;
-      for (int base = 0; base < nodes * G; base += blockDim.x) {
-         const int idx = base + t;
-         const int n = idx / G, part = idx - (idx / G) * G;
-         T m = T(0);
-         if (n < nodes)
-            for (int b = part; b < A; b += G) m += (REV ? T(1) : ws[b]) * xs[n * A + b];
-         m += __shfl_xor_sync(0xffffffffu, m, 1);
-         m += __shfl_xor_sync(0xffffffffu, m, 2);
-         if (part == 0 && n < nodes) mom[n] = m * ssw[n / NB];
+      // Stage: the block's own rows (one contiguous range), each cell's class
+      // record and this thread's upwind runs, all in flight at once (with the
+      // ring, the first two faces' runs, each in a commit group of its own).
+      // Per face 4 bits of fcode: 8 for an interior face, else the boundary side.
+      unsigned fcode = 0;
+      {
+         const int nu = kc * NB * A * (int)sizeof(T) / CU;
+         const unsigned char *src = reinterpret_cast<const unsigned char *>(x + c0 * NB * A);
+         for (int u = t; u < nu; u += blockDim.x) CpAsyncRun<CU>(reinterpret_cast<unsigned char *>(xs) + u * CU, src + u * CU);
       }
-   }
-
-   T acc[AP][NB];
-   if (live) {
-      const T *r = recs + k * L.size;
-      const T *xk = xs + k * NB * A;
-      constexpr int TS = L.size - L.tail;  // grad phi and 1 / V
-      T tl[TS];
-      LoadShared<T, TS>(r + L.tail, tl);
-      T xo[AP][NB];
+      if (live) {
+         const T *rec = g.rec + (int64_t)cls * L.size;
+         for (int u = q; u < RU; u += QA) CpAsync<16>(recs + k * L.size + u * (16 / (int)sizeof(T)), rec + u * (16 / (int)sizeof(T)));
+         if constexpr (kRing) CpAsyncCommit();
+         T vc = T(0);
+         if constexpr (REV) vc = g.volume[c];
 #pragma unroll
-      for (int j = 0; j < NB; j++) {
-         T v[AP];
-         LoadShared<T, AP>(xk + j * A + ar0, v);
-#pragma unroll
-         for (int p = 0; p < AP; p++) xo[p][j] = REV ? v[AP - 1 - p] : v[p];
-      }
-      // Removal, and the volume term -(Omega . grad phi_i) x(c, 0, a) for i > 0
-#pragma unroll
-      for (int p = 0; p < AP; p++)
-#pragma unroll
-         for (int i = 0; i < NB; i++) acc[p][i] = sig_t * xo[p][i];
-      if constexpr (NB > 1) {
-#pragma unroll
-         for (int i = 1; i < NB; i++)
-#pragma unroll
-            for (int p = 0; p < AP; p++) acc[p][i] -= Dot3(om + 3 * p, tl + 3 * i) * xo[p][0];
-      }
-      // Each face without a branch on the sign of s = Omega . nA: outflow
-      // max(s, 0) face_own x, inflow min(s, 0) face_up x_up, x_up the
-      // neighbour, this cell's mirrored ordinate on a reflective side, zero
-      // on a vacuum side (DG0: the same with 1 / V for both matrices). DG1:
-      // unrolled, with the faces' reads kept apart (hoisted together they
-      // would spill), so that no index is formed at run time: 256^2 triangles
-      // S8 140 -> 129 us FP64, 48^3 hexahedra 434 -> 404 FP64, 224 -> 205
-      // FP32. DG0, whose faces are a few instructions, is faster in a loop
-      // (unscattered 256^2 triangles 48 us against 54)
-#pragma unroll (NB > 1 ? F : 1)
-      for (int f = 0; f < F; f++) {
-         if constexpr (NB > 1) asm volatile("" ::: "memory");
-         const unsigned fc = (fcode >> (4 * f)) & 15u;
-         T na[4];
-         LoadShared<T, 4>(r + L.nA(f), na);
-         T xn[AP][NB];
-         const int slot = kRing ? (f & 1) : f;
-         if constexpr (kRing) {
-            // This face's group is in once at most the next face's is pending
-            if (f + 1 < F) CpAsyncWaitGroup<1>();
-            else CpAsyncWaitGroup<0>();
-         }
-         if (fc & 8u) {
-#pragma unroll
-            for (int j = 0; j < NB; j++) {
-               T v[AP];
-               LoadShared<T, AP>(xup + ((slot * NB + j) * (int)blockDim.x + t) * AP, v);
-#pragma unroll
-               for (int p = 0; p < AP; p++) xn[p][j] = REV ? v[AP - 1 - p] : v[p];
-            }
-         } else {
-            const int side = (int)fc;
-            const bool refl = g.side_bc[side] == UBOLT_BC_REFLECT;
-#pragma unroll
-            for (int p = 0; p < AP; p++) {
-               int ar = refl ? g.refl[(side >> 1) * A + a0 + p] : 0;
-               if (REV && refl) ar = g.opp[ar];
-#pragma unroll
-               for (int j = 0; j < NB; j++) xn[p][j] = refl ? xk[j * A + ar] : T(0);
-            }
-         }
-         T sp[AP], sm[AP];
-         const T ratio = (REV && (fc & 8u)) ? rat[f * (int)blockDim.x + t] : T(1);
-#pragma unroll
-         for (int p = 0; p < AP; p++) {
-            const T s = Dot3(om + 3 * p, na);
-            sp[p] = fmax(s, T(0));
-            sm[p] = fmin(s, T(0));
-            if constexpr (REV) sm[p] *= ratio;
-         }
-         if constexpr (NB == 1) {
-#pragma unroll
-            for (int p = 0; p < AP; p++) acc[p][0] += (sp[p] * xo[p][0] + sm[p] * xn[p][0]) * tl[0];
-         } else {
-            {
-               T m[L.fm];
-               LoadShared<T, L.fm>(r + L.fown(f), m);
-#pragma unroll
-               for (int p = 0; p < AP; p++)
-#pragma unroll
-                  for (int i = 0; i < NB; i++) {
-                     T u = T(0);
-#pragma unroll
-                     for (int j = 0; j < NB; j++) u += m[i * NB + j] * xo[p][j];
-                     acc[p][i] += sp[p] * u;
-                  }
-            }
-            {
-               T m[L.fm];
-               LoadShared<T, L.fm>(r + L.fup(f), m);
-#pragma unroll
-               for (int p = 0; p < AP; p++)
-#pragma unroll
-                  for (int i = 0; i < NB; i++) {
-                     T v = T(0);
-#pragma unroll
-                     for (int j = 0; j < NB; j++) v += m[i * NB + j] * xn[p][j];
-                     acc[p][i] += sm[p] * v;
-                  }
-            }
-         }
-         if constexpr (kRing) {
-            // This face's runs are used: fetch face f + 2's into the slot
-            if (f + XS < F) {
-               const int32_t cf = g.code[c * F + f + XS];
-               if (FaceInterior(cf)) {
+         for (int f = 0; f < F; f++) {
+            const int32_t cf = code[f];
+            if (FaceInterior(cf)) {
+               fcode |= 8u << (4 * f);
+               if constexpr (REV) rat[f * (int)blockDim.x + t] = vc * g.inv_vol[g.cls[cf]];
+               if (!kRing || f < XS) {
 #pragma unroll
                   for (int j = 0; j < NB; j++)
-                     CpAsyncRun<CU>(xup + ((slot * NB + j) * (int)blockDim.x + t) * AP, x + ((int64_t)cf * NB + j) * A + ar0);
+                     CpAsyncRun<CU>(xup + ((f * NB + j) * (int)blockDim.x + t) * AP, x + ((int64_t)cf * NB + j) * A + ar0);
+               }
+            } else {
+               fcode |= (unsigned)FaceSide(cf) << (4 * f);
+            }
+            if (kRing && f < XS) CpAsyncCommit();
+         }
+      }
+      T sig_t = T(0);
+      if (live) {
+         if constexpr (!kRounds) LoadRun<T, 3 * AP>(g.omega + 3 * a0, om);
+         sig_t = g.sigma_t[c];
+         if (SCATTER && q == 0) ssw[k] = g.sigma_s[c] * g.inv_sum_weights;
+      }
+      if constexpr (SCATTER && !kRounds)
+         for (int b = t; b < A; b += blockDim.x) ws[b] = g.w[b];
+      // The shared rows and records are in; with the ring, a live thread's two
+      // face groups may still be in flight (a thread without a cell committed
+      // no group, so it waits for all of its copies)
+      if (kRing && live) CpAsyncWaitGroup<XS>();
+      else CpAsyncWaitAll();
+      __syncthreads();
+
+      if constexpr (SCATTER) {
+         // sigma_s / W sum_b w_b x(node, b) from the staged rows: four lanes
+         // per node, each a fixed quarter of the ordinates, then two shuffles.
+         // The loop bound is the same for every thread (the shuffles need the
+         // whole warp).
+         constexpr int G = 4;
+         const int nodes = kc * NB;
+         for (int base = 0; base < nodes * G; base += blockDim.x) {
+            const int idx = base + t;
+            const int n = idx / G, part = idx - (idx / G) * G;
+            T m = T(0);
+            if (n < nodes)
+               for (int b = part; b < A; b += G) m += (REV ? T(1) : ws[b]) * xs[n * A + b];
+            m += __shfl_xor_sync(0xffffffffu, m, 1);
+            m += __shfl_xor_sync(0xffffffffu, m, 2);
+            if (part == 0 && n < nodes) mom[n] = m * ssw[n / NB];
+         }
+      }
+
+      T acc[AP][NB];
+      if (live) {
+         const T *r = recs + k * L.size;
+         const T *xk = xs + k * NB * A;
+         constexpr int TS = L.size - L.tail;  // grad phi and 1 / V
+         T tl[TS];
+         LoadShared<T, TS>(r + L.tail, tl);
+         T xo[AP][NB];
+#pragma unroll
+         for (int j = 0; j < NB; j++) {
+            T v[AP];
+            LoadShared<T, AP>(xk + j * A + ar0, v);
+#pragma unroll
+            for (int p = 0; p < AP; p++) xo[p][j] = REV ? v[AP - 1 - p] : v[p];
+         }
+         // Removal, and the volume term -(Omega . grad phi_i) x(c, 0, a) for i > 0
+#pragma unroll
+         for (int p = 0; p < AP; p++)
+#pragma unroll
+            for (int i = 0; i < NB; i++) acc[p][i] = sig_t * xo[p][i];
+         if constexpr (NB > 1) {
+#pragma unroll
+            for (int i = 1; i < NB; i++)
+#pragma unroll
+               for (int p = 0; p < AP; p++) acc[p][i] -= Dot3(om + 3 * p, tl + 3 * i) * xo[p][0];
+         }
+         // Each face without a branch on the sign of s = Omega . nA: outflow
+         // max(s, 0) face_own x, inflow min(s, 0) face_up x_up, x_up the
+         // neighbour, this cell's mirrored ordinate on a reflective side, zero
+         // on a vacuum side (DG0: the same with 1 / V for both matrices). DG1:
+         // unrolled, with the faces' reads kept apart (hoisted together they
+         // would spill), so that no index is formed at run time: 256^2 triangles
+         // S8 140 -> 129 us FP64, 48^3 hexahedra 434 -> 404 FP64, 224 -> 205
+         // FP32. DG0, whose faces are a few instructions, is faster in a loop
+         // (unscattered 256^2 triangles 48 us against 54)
+#pragma unroll (NB > 1 ? F : 1)
+         for (int f = 0; f < F; f++) {
+            if constexpr (NB > 1) asm volatile("" ::: "memory");
+            const unsigned fc = (fcode >> (4 * f)) & 15u;
+            T na[4];
+            LoadShared<T, 4>(r + L.nA(f), na);
+            T xn[AP][NB];
+            const int slot = kRing ? (f & 1) : f;
+            if constexpr (kRing) {
+               // This face's group is in once at most the next face's is pending
+               if (f + 1 < F) CpAsyncWaitGroup<1>();
+               else CpAsyncWaitGroup<0>();
+            }
+            if (fc & 8u) {
+#pragma unroll
+               for (int j = 0; j < NB; j++) {
+                  T v[AP];
+                  LoadShared<T, AP>(xup + ((slot * NB + j) * (int)blockDim.x + t) * AP, v);
+#pragma unroll
+                  for (int p = 0; p < AP; p++) xn[p][j] = REV ? v[AP - 1 - p] : v[p];
+               }
+            } else {
+               const int side = (int)fc;
+               const bool refl = g.side_bc[side] == UBOLT_BC_REFLECT;
+#pragma unroll
+               for (int p = 0; p < AP; p++) {
+                  int ar = refl ? g.refl[(side >> 1) * A + a0 + p] : 0;
+                  if (REV && refl) ar = g.opp[ar];
+#pragma unroll
+                  for (int j = 0; j < NB; j++) xn[p][j] = refl ? xk[j * A + ar] : T(0);
                }
             }
-            CpAsyncCommit();
+            T sp[AP], sm[AP];
+            const T ratio = (REV && (fc & 8u)) ? rat[f * (int)blockDim.x + t] : T(1);
+#pragma unroll
+            for (int p = 0; p < AP; p++) {
+               const T s = Dot3(om + 3 * p, na);
+               sp[p] = fmax(s, T(0));
+               sm[p] = fmin(s, T(0));
+               if constexpr (REV) sm[p] *= ratio;
+            }
+            if constexpr (NB == 1) {
+#pragma unroll
+               for (int p = 0; p < AP; p++) acc[p][0] += (sp[p] * xo[p][0] + sm[p] * xn[p][0]) * tl[0];
+            } else {
+               {
+                  T m[L.fm];
+                  LoadShared<T, L.fm>(r + L.fown(f), m);
+#pragma unroll
+                  for (int p = 0; p < AP; p++)
+#pragma unroll
+                     for (int i = 0; i < NB; i++) {
+                        T u = T(0);
+#pragma unroll
+                        for (int j = 0; j < NB; j++) u += m[i * NB + j] * xo[p][j];
+                        acc[p][i] += sp[p] * u;
+                     }
+               }
+               {
+                  T m[L.fm];
+                  LoadShared<T, L.fm>(r + L.fup(f), m);
+#pragma unroll
+                  for (int p = 0; p < AP; p++)
+#pragma unroll
+                     for (int i = 0; i < NB; i++) {
+                        T v = T(0);
+#pragma unroll
+                        for (int j = 0; j < NB; j++) v += m[i * NB + j] * xn[p][j];
+                        acc[p][i] += sm[p] * v;
+                     }
+               }
+            }
+            if constexpr (kRing) {
+               // This face's runs are used: fetch face f + 2's into the slot
+               if (f + XS < F) {
+                  const int32_t cf = g.code[c * F + f + XS];
+                  if (FaceInterior(cf)) {
+#pragma unroll
+                     for (int j = 0; j < NB; j++)
+                        CpAsyncRun<CU>(xup + ((slot * NB + j) * (int)blockDim.x + t) * AP, x + ((int64_t)cf * NB + j) * A + ar0);
+                  }
+               }
+               CpAsyncCommit();
+            }
          }
       }
-   }
-   if constexpr (SCATTER) {
-      __syncthreads();
+      // Also: all threads are done with the staged rows and records, which the next
+      // round's copies replace (the node moments only after that round's barrier)
+      if constexpr (SCATTER || kRounds) __syncthreads();
+      if constexpr (SCATTER) {
+         if (live) {
+#pragma unroll
+            for (int p = 0; p < AP; p++) {
+               const T wa = REV ? ws[a0 + p] : T(1);  // the transpose: w of the row's own ordinate (w_opp = w)
+#pragma unroll
+               for (int i = 0; i < NB; i++) acc[p][i] -= wa * mom[k * NB + i];
+            }
+         }
+      }
       if (live) {
 #pragma unroll
-         for (int p = 0; p < AP; p++) {
-            const T wa = REV ? ws[a0 + p] : T(1);  // the transpose: w of the row's own ordinate (w_opp = w)
+         for (int i = 0; i < NB; i++) {
+            T v[AP];
 #pragma unroll
-            for (int i = 0; i < NB; i++) acc[p][i] -= wa * mom[k * NB + i];
+            for (int p = 0; p < AP; p++) v[REV ? AP - 1 - p : p] = acc[p][i];
+            StoreRun<T, AP>(y + (c * NB + i) * A + ar0, v);
          }
       }
-   }
-   if (!live) return;
-#pragma unroll
-   for (int i = 0; i < NB; i++) {
-      T v[AP];
-#pragma unroll
-      for (int p = 0; p < AP; p++) v[REV ? AP - 1 - p : p] = acc[p][i];
-      StoreRun<T, AP>(y + (c * NB + i) * A + ar0, v);
+      if constexpr (!kRounds) return;
    }
 }
 
@@ -463,12 +494,12 @@ __global__ void DiagonalKernel(const DevGeom<T> g, T *__restrict__ d)
 // Cells per block for QA threads per cell: the most live threads resident
 // per SM for this kernel (registers and shared memory), then the fewest idle
 // lanes, then the most blocks per SM (more blocks stage their copies
-// independently). Cached per kernel and QA.
+// independently). With them the blocks per SM. Cached per kernel and QA.
 template <typename Kern, typename Smem>
-static int ApplyCells(Kern kern, int QA, Smem smem_of)
+static std::pair<int, int> ApplyCells(Kern kern, int QA, Smem smem_of)
 {
    static std::mutex mu;
-   static std::map<std::pair<const void *, int>, int> memo;
+   static std::map<std::pair<const void *, int>, std::pair<int, int>> memo;
    const auto key = std::make_pair(reinterpret_cast<const void *>(kern), QA);
    {
       std::lock_guard<std::mutex> lk(mu);
@@ -506,8 +537,7 @@ static int ApplyCells(Kern kern, int QA, Smem smem_of)
       }
    }
    std::lock_guard<std::mutex> lk(mu);
-   memo[key] = best;
-   return best;
+   return memo[key] = {best, std::max(best_blocks, 1)};
 }
 
 // True where the opposite maps every aligned run of ap ordinates onto an
@@ -551,8 +581,8 @@ int LaunchApply(const ubolt_ctx *ctx, const DevGeom<T> &g, const T *x, T *y, int
          return sizeof(T) * (vec ? ApplySmemElems<T, NB, F, AV>(K, thr, A, rev)
                                  : ApplySmemElems<T, NB, F, 1>(K, thr, A, rev));
       };
-      const int Kt = ApplyCells(kern, QA, smem_of);
-      const int64_t nblk = (g.n_cells + Kt - 1) / Kt;
+      const auto [Kt, per_sm] = ApplyCells(kern, QA, smem_of);
+      int64_t nblk = (g.n_cells + Kt - 1) / Kt;
       const int nthr = (Kt * QA + 31) / 32 * 32;
       const size_t smem = smem_of(Kt, nthr);
       if (smem > 48 * 1024) {
@@ -562,6 +592,12 @@ int LaunchApply(const ubolt_ctx *ctx, const DevGeom<T> &g, const T *x, T *y, int
             return SetError(UBOLT_ERR_ARG, "apply: %zu bytes of shared memory for %d ordinates: %s", smem, g.A,
                             cudaGetErrorString(e));
          }
+      }
+      if (vec && ApplyRounds<NB, F, AV>()) {
+         int dev = 0, n_sm = 0;
+         cudaGetDevice(&dev);
+         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+         nblk = std::min<int64_t>(nblk, (int64_t)per_sm * std::max(n_sm, 1));
       }
       kern<<<nblk, nthr, smem, s>>>(g, x, y, Kt);
    }
