@@ -50,7 +50,8 @@ struct ubolt_solver {
    bool flexible = false;
    double *Z = nullptr;
    float *Z32 = nullptr;
-   // Reductions: partial[red_blocks][restart + 2], h[3 * (restart + 2)]
+   // Reductions: partial[red_blocks][restart + 2] (the Gram-Schmidt kernel's:
+   // two sets of [gs_blocks][restart + 2]), h[3 * (restart + 2)]
    double *partial = nullptr, *h = nullptr;
    int red_blocks = 0, gs_blocks = 0;
    // [0] the multi-dot's finished-block counter, zero between launches; [1] the
@@ -93,6 +94,10 @@ constexpr int kChunk = 8;
 // stops). The two passes' h, |phi_w|^2 and alpha_w before the division go to
 // the mailbox, from which the host forms the Hessenberg column. Every block
 // adds all blocks' shares itself, in one order, so all hold the same scalars.
+// The shares of reduction k (pass 0, pass 1, the norm) go to set k % 2: a
+// block writes set k % 2 again, for reduction k + 2, only after barrier k + 1,
+// on which every block arrives after it has read the shares of reduction k.
+// (In one set a block ahead would write over shares still being read.)
 // Bound by the barriers (about 2 us each with the sums) and, for long vectors, by
 // 4 (j + 2) n_nodes 8 bytes through L2. As eight launches a step (dots, updates,
 // scaling) 256^2 triangles (393 k nodes) took about 60 us, now 34; a whole solve
@@ -108,7 +113,7 @@ struct GsArgs {
    int j1;
    double *alpha;  // [j1 + 1]; [j1] written
    double rp2, kappa;
-   double *partial;  // [blocks][stride]
+   double *partial;  // [2][blocks][stride]
    int stride;
    unsigned *count;
    unsigned base;  // the counter's value at launch
@@ -123,23 +128,26 @@ __global__ void __launch_bounds__(kGsThreads, kGsBlocksPerSm) GramSchmidtKernel(
    __shared__ int ok;
    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, G = gridDim.x, j1 = a.j1;
    const int64_t first = (int64_t)blockIdx.x * kGsThreads + t, step = (int64_t)G * kGsThreads;
-   unsigned barriers = 0;
+   unsigned reduction = 0;  // its number, the same in every thread
    for (int i = t; i < j1; i += kGsThreads) al[i] = a.alpha[i];
    if (t == 0) ok = 1;
    __syncthreads();
    if (t == 0) aw = al[j1 - 1];
+   // Block b's shares of the current reduction
+   auto shares = [&](int b) { return a.partial + ((int64_t)(reduction & 1) * G + b) * a.stride; };
    // h[i] = the sum over the grid of every block's share of value i
    auto grid_sum = [&](int n_values) {
       __syncthreads();
-      if (t == 0) ok = GridArrive(a.count, a.base + ++barriers * (unsigned)G) && ok;
+      if (t == 0) ok = GridArrive(a.count, a.base + (reduction + 1) * (unsigned)G) && ok;
       __syncthreads();
       for (int i = warp; i < n_values; i += kWarps) {
          double s = 0.0;
-         for (int b = lane; b < G; b += 32) s += __ldcg(a.partial + (int64_t)b * a.stride + i);
+         for (int b = lane; b < G; b += 32) s += __ldcg(shares(b) + i);
 #pragma unroll
          for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
          if (lane == 0) h[i] = s;
       }
+      reduction++;
       __syncthreads();
    };
    // The block's shares of nc values held by its threads, from value i0
@@ -155,7 +163,7 @@ __global__ void __launch_bounds__(kGsThreads, kGsBlocksPerSm) GramSchmidtKernel(
       if (t < nc) {
          double s = 0.0;
          for (int w = 0; w < kWarps; w++) s += red[t][w];
-         a.partial[(int64_t)blockIdx.x * a.stride + i0 + t] = s;
+         shares(blockIdx.x)[i0 + t] = s;
       }
       __syncthreads();
    };
@@ -1095,7 +1103,7 @@ static int EnsureWorkspace(ubolt_ctx *ctx, const ubolt_solve_options *o)
    int rc = 0;
    ctx->solver = ws;
    if ((rc = alloc((void **)&ws->r, n * 8)) || (rc = alloc((void **)&ws->z, n * 8)) ||
-       (rc = alloc((void **)&ws->t, n * 8)) || (rc = alloc((void **)&ws->partial, (size_t)std::max(ws->red_blocks, ws->gs_blocks) * (m + 2) * 8)) ||
+       (rc = alloc((void **)&ws->t, n * 8)) || (rc = alloc((void **)&ws->partial, (size_t)std::max(ws->red_blocks, 2 * ws->gs_blocks) * (m + 2) * 8)) ||
        (rc = alloc((void **)&ws->h, 3 * (size_t)(m + 2) * 8)))
       return rc;
    if ((rc = alloc((void **)&ws->md_count, 16))) return rc;
