@@ -612,6 +612,12 @@ int ubolt_solve_host_batch(ubolt_ctx *ctx, int n, const double *const *b_host, d
  * returns as ubolt_solve. */
 int ubolt_solve_adjoint(ubolt_ctx *ctx, const double *g, double *lambda, const ubolt_solve_options *opts,
                         ubolt_solve_stats *stats, void *stream);
+/* Failure-path check of the bounded waits of the compressed basis's
+ * orthogonalisation (no reference counterpart): set the wait limit in polls
+ * (default 2^24), and with unmet_block >= 0 make that block of the NEXT step
+ * wait for arrivals that never come. That solve returns UBOLT_ERR_TIMEOUT, and
+ * later solves are normal again. Needs a solver set up without a DSA stage. */
+int ubolt_solve_test_wait(ubolt_ctx *ctx, uint32_t spin_limit, int unmet_block);
 /* g(c, 0, a) += detector(c) V_c w_a: the adjoint source of the response
  * J = sum_c detector(c) V_c phi(c, 0) = g^T psi (detector: device, n_cells). */
 int ubolt_add_response_source(ubolt_ctx *ctx, const double *detector, double *g, void *stream);

@@ -75,3 +75,20 @@ def test_the_solves_above_need_long_bases():
     x, s = T.TransportSolver(ctx, rtol=1e-9, restart=200, max_it=400).solve(b)
     assert s["krylov"] == 2 and s["iterations"] > 33
     ctx.close()
+
+
+@pytest.mark.parametrize("block", [0, 7, 35])
+def test_a_wait_that_gives_up_fails_the_solve(block):
+    """Whichever block's wait runs out, the solve reports it, and the next
+    one is as before."""
+    ctx, keep, b = diffusive("many_blocks")
+    solver = T.TransportSolver(ctx, rtol=1e-9, restart=200, max_it=400)
+    ref, s = solver.solve(b)
+    T._lib.check(T.lib.ubolt_solve_test_wait(ctx.handle, 2000, block))
+    with pytest.raises(T._lib.UboltError) as e:
+        solver.solve(b)
+    assert e.value.status == 6  # UBOLT_ERR_TIMEOUT
+    T._lib.check(T.lib.ubolt_solve_test_wait(ctx.handle, 1 << 24, -1))
+    x, s2 = solver.solve(b)
+    assert torch.equal(x, ref) and s2["iterations"] == s["iterations"]
+    ctx.close()

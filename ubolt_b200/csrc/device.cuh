@@ -571,15 +571,16 @@ __device__ __forceinline__ void CellFactors(const T *rec, T sigma_t, const T om[
 // A grid barrier's arrival and wait, by one thread of a block of a cooperative
 // launch: the block's writes so far are released, `target` arrivals waited for
 // (the blocks' number times the barriers so far), the others' writes acquired.
-// Bounded; false: gave up. The fence empties the SM's L1.
-__device__ __forceinline__ bool GridArrive(unsigned *count, unsigned target)
+// Bounded, at most limit + 1 polls; false: gave up. The fence empties the SM's L1.
+constexpr uint32_t kGridSpins = 1u << 24;
+__device__ __forceinline__ bool GridArrive(unsigned *count, unsigned target, uint32_t limit = kGridSpins)
 {
    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
    unsigned v;
    uint32_t tries = 0;
    do {
       asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-   } while ((int)(v - target) < 0 && ++tries < (1u << 24));
+   } while ((int)(v - target) < 0 && tries++ < limit);
    __threadfence();
    return (int)(v - target) >= 0;
 }

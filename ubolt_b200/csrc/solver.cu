@@ -54,6 +54,10 @@ struct ubolt_solver {
    // two sets of [gs_blocks][restart + 2]), h[3 * (restart + 2)]
    double *partial = nullptr, *h = nullptr;
    int red_blocks = 0, gs_blocks = 0;
+   // The Gram-Schmidt kernel's waits: polls before one gives up, and (a test
+   // hook, for one step) the block whose waits cannot be met, or -1
+   uint32_t gs_spin_limit = ubolt::kGridSpins;
+   int gs_unmet_block = -1;
    // [0] the multi-dot's finished-block counter, zero between launches; [1] the
    // Gram-Schmidt kernel's barrier counter
    unsigned *md_count = nullptr;
@@ -117,7 +121,11 @@ struct GsArgs {
    int stride;
    unsigned *count;
    unsigned base;  // the counter's value at launch
-   double *box_h1, *box_h2, *box_alpha;  // mailbox: h1[j1], h2[j1 + 1] (last |phi_w|^2), alpha_w
+   uint32_t spin_limit;
+   int unmet_block;
+   // Mailbox: h1[j1], h2[j1 + 1] (last |phi_w|^2), alpha_w, and the fault word,
+   // set by any block whose wait gave up (the vectors are then not valid)
+   double *box_h1, *box_h2, *box_alpha, *box_fault;
 };
 
 __global__ void __launch_bounds__(kGsThreads, kGsBlocksPerSm) GramSchmidtKernel(const GsArgs a)
@@ -138,7 +146,15 @@ __global__ void __launch_bounds__(kGsThreads, kGsBlocksPerSm) GramSchmidtKernel(
    // h[i] = the sum over the grid of every block's share of value i
    auto grid_sum = [&](int n_values) {
       __syncthreads();
-      if (t == 0) ok = GridArrive(a.count, a.base + (reduction + 1) * (unsigned)G) && ok;
+      if (t == 0) {
+         // After a wait that gave up the block still arrives, and waits no more
+         const unsigned target = a.base + (reduction + 1) * (unsigned)G;
+         const unsigned never = (int)blockIdx.x == a.unmet_block ? 1u << 30 : 0u;
+         if (!GridArrive(a.count, target + never, ok ? a.spin_limit : 0u) && ok) {
+            ok = 0;
+            *a.box_fault = 1.0;
+         }
+      }
       __syncthreads();
       for (int i = warp; i < n_values; i += kWarps) {
          double s = 0.0;
@@ -211,7 +227,7 @@ __global__ void __launch_bounds__(kGsThreads, kGsBlocksPerSm) GramSchmidtKernel(
    }
    grid_sum(1);
    if (t == 0) {
-      const double phi2 = ok ? h[0] : __longlong_as_double(0x7ff8000000000000LL);  // gave up: the host stops
+      const double phi2 = h[0];
       // Rounded step by step (no fused multiply-add), as the host's expression is
       const double hn = sqrt(__dadd_rn(__dmul_rn(__dmul_rn(aw, aw), a.rp2), __dmul_rn(a.kappa, phi2)));
       const bool good = hn > 0.0 && isfinite(hn);
@@ -381,7 +397,7 @@ __global__ void MailCopyKernel(const double *__restrict__ src, double *__restric
 }
 
 // Mailbox offsets (doubles) in each half
-constexpr int kMbScalars = 0, kMbH1 = 8;
+constexpr int kMbScalars = 0, kMbFault = 7, kMbH1 = 8;
 
 // n device values to the mailbox at off; read ws->mb_h[off ...] after the stream syncs
 static void ToHost(const ubolt_solver *ws, const double *dev, int off, int n, cudaStream_t s)
@@ -422,7 +438,7 @@ static void ToDevice(const ubolt_solver *ws, const double *host, double *dev, in
 // One Gram-Schmidt step of the compressed basis (see GramSchmidtKernel): w
 // against Phi[0 .. j1), scalars in alpha, the Hessenberg column to the mailbox.
 // *base: the barrier counter's value, advanced by the launch's arrivals.
-static int GramSchmidt(const ubolt_solver *ws, const double *Phi, int j1, double *w, double *alpha, double rp2,
+static int GramSchmidt(ubolt_solver *ws, const double *Phi, int j1, double *w, double *alpha, double rp2,
                        double kappa, unsigned *base, cudaStream_t s)
 {
    int dev = 0, sms = 0, per_sm = 0;
@@ -446,6 +462,10 @@ static int GramSchmidt(const ubolt_solver *ws, const double *Phi, int j1, double
    a.box_h1 = ws->mb_d + kMbH1;
    a.box_h2 = ws->mb_d + kMbH1 + (ws->restart + 2);
    a.box_alpha = ws->mb_d + kMbScalars;
+   a.box_fault = ws->mb_d + kMbFault;
+   a.spin_limit = ws->gs_spin_limit;
+   a.unmet_block = ws->gs_unmet_block;
+   ws->gs_unmet_block = -1;
    void *params[] = {&a};
    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)GramSchmidtKernel, dim3(grid), dim3(kGsThreads), params,
                                                      0, s);
@@ -911,7 +931,7 @@ static int IsoGrid(int64_t n_nodes)
 }
 
 template <typename S>
-static int GmresIso(ubolt_ctx *ctx, const ubolt_solver *ws, S *work, const S *b, S *x, double bnorm, double rtol,
+static int GmresIso(ubolt_ctx *ctx, ubolt_solver *ws, S *work, const S *b, S *x, double bnorm, double rtol,
                     int max_it, bool adjoint, bool x_zero, GmresResult *out, void *stream)
 {
    cudaStream_t s = (cudaStream_t)stream;
@@ -942,6 +962,7 @@ static int GmresIso(ubolt_ctx *ctx, const ubolt_solver *ws, S *work, const S *b,
    int rc = 0;
    // The Gram-Schmidt kernel's barrier counter starts every system at zero
    unsigned gs_base = 0;
+   ws->mb_h[kMbFault] = 0.0;
    if ((rc = CudaCheck(cudaMemsetAsync(ws->md_count + 1, 0, sizeof(unsigned), s), "gmres"))) return rc;
    out->iterations = 0;
    out->converged = false;
@@ -1005,6 +1026,8 @@ static int GmresIso(ubolt_ctx *ctx, const ubolt_solver *ws, S *work, const S *b,
          // waits on nothing the host sends
          if ((rc = GramSchmidt(ws, Phi, j + 1, pn, alpha, rp2, kappa, &gs_base, s))) return rc;
          if ((rc = CudaCheck(cudaStreamSynchronize(s), "gmres"))) return rc;
+         if (ws->mb_h[kMbFault] != 0.0)
+            return SetError(UBOLT_ERR_TIMEOUT, "a wait of the orthogonalisation gave up at iteration %d", out->iterations + 1);
          std::copy(ws->mb_h + kMbH1, ws->mb_h + kMbH1 + j + 1, h1.begin());
          std::copy(ws->mb_h + kMbH1 + (m + 2), ws->mb_h + kMbH1 + (m + 2) + j + 2, h2.begin());
          alpha_h[j + 1] = ws->mb_h[kMbScalars];
@@ -1369,4 +1392,15 @@ extern "C" int ubolt_solve_adjoint(ubolt_ctx *ctx, const double *g, double *lamb
                                    ubolt_solve_stats *stats, void *stream)
 {
    return SolveSystem(ctx, true, g, lambda, opts, stats, stream);
+}
+
+extern "C" int ubolt_solve_test_wait(ubolt_ctx *ctx, uint32_t spin_limit, int unmet_block)
+{
+   int rc = CheckReady(ctx, false);
+   if (rc) return rc;
+   if (spin_limit < 16) return SetError(UBOLT_ERR_ARG, "spin limit %u too small", spin_limit);
+   if (!ctx->solver || !ctx->solver->Phi) return SetError(UBOLT_ERR_STATE, "no solver with a compressed basis");
+   ctx->solver->gs_spin_limit = spin_limit;
+   ctx->solver->gs_unmet_block = unmet_block;
+   return UBOLT_OK;
 }
