@@ -31,13 +31,11 @@ struct OwnRecord {
 // B r = x solved in place by Gaussian elimination with partial pivoting,
 // without a branch: the largest entry of a column is brought up by
 // conditional row swaps (each row is eliminated by the same arithmetic
-// wherever it stands), and a quotient s / b is s (1 / b) corrected once by its
-// remainder, which rounds as the division does but for the last place. A zero
-// pivot (a singular block) gives zero, as its zeroed inverse does in the reference.
+// wherever it stands). A zero pivot (a singular block) gives zero, as its
+// zeroed inverse does in the reference.
 template <typename T, int NB>
 __device__ __forceinline__ void SolveBlockSelect(T B[NB][NB], T r[NB])
 {
-   T inv[NB];
    bool singular = false;
 #pragma unroll
    for (int k = 0; k < NB; k++) {
@@ -55,10 +53,10 @@ __device__ __forceinline__ void SolveBlockSelect(T B[NB][NB], T r[NB])
          r[i] = up ? a : b;
       }
       singular |= B[k][k] == T(0);
-      inv[k] = T(1) / B[k][k];
+      const T inv = T(1) / B[k][k];
 #pragma unroll
       for (int i = k + 1; i < NB; i++) {
-         const T f = B[i][k] * inv[k];
+         const T f = B[i][k] * inv;
 #pragma unroll
          for (int j = k + 1; j < NB; j++) B[i][j] -= f * B[k][j];
          r[i] -= f * r[k];
@@ -69,9 +67,7 @@ __device__ __forceinline__ void SolveBlockSelect(T B[NB][NB], T r[NB])
       T s = r[k];
 #pragma unroll
       for (int j = k + 1; j < NB; j++) s -= B[k][j] * r[j];
-      const T q = s * inv[k];
-      const T rem = fma(-q, B[k][k], s), better = fma(rem, inv[k], q);
-      r[k] = isfinite(better) ? better : q;  // (an infinite quotient has no remainder)
+      r[k] = s / B[k][k];
    }
    if (singular)
 #pragma unroll
