@@ -168,3 +168,12 @@ def test_dg1_zero_pivot_gives_zero(off):
                                          offset_copy(torch.full((ctx.n_rows,), 5.0, dtype=torch.float32), off))
     assert bool((y == 0).all())
     ctx.close()
+
+
+@pytest.mark.parametrize("sn", [4, 8, 12, 16])
+@pytest.mark.parametrize("order", [0, 1])
+@pytest.mark.parametrize("shape", MESHES)
+def test_block_shapes_match_oracle(shape, order, sn):
+    """Ordinate counts that make blocks of 96 to 160 threads, of one cell to
+    dozens, and a cell walked in rounds."""
+    test_block_apply_matches_oracle(shape, order, sn)

@@ -17,8 +17,11 @@ template <typename T, int NB, int F>
 struct OwnRecord {
    static constexpr RecordLayout L = RecordLayout(NB, F, (int)sizeof(T));
    static constexpr int kUnit = 16 / (int)sizeof(T);
-   static constexpr int kFace = 4 + L.fm, kTail = F * kFace, kSize = kTail + L.size - L.tail;
-   static constexpr int kFaceUnits = kFace / kUnit, kUnits = kSize / kUnit;
+   static constexpr int kFace = 4 + L.fm, kTail = F * kFace;
+   static constexpr int kFaceUnits = kFace / kUnit, kUnits = (kTail + L.size - L.tail) / kUnit;
+   // The stride between records, odd in 16-byte units: lanes of different
+   // cells then read different banks
+   static constexpr int kSize = (kUnits | 1) * kUnit;
    // Unit u's place in the class record
    static __device__ __forceinline__ int Source(int u)
    {
@@ -74,23 +77,23 @@ __device__ __forceinline__ void SolveBlockSelect(T B[NB][NB], T r[NB])
       for (int k = 0; k < NB; k++) r[k] = T(0);
 }
 
-constexpr int kBlockThreads = 128;
-// Blocks per SM the registers should leave room for: all that fit without
-// spilling (256^2 triangles, FP64: 97 us at five, 87 at six, 82 at eight; blocks
-// of 256 threads 123)
+// Most threads of a block (see BlockApplyShape)
+constexpr int kBlockThreads = 160;
+// Blocks of that many per SM the registers should leave room for: all that fit
+// without heavy spills (256^2 triangles, FP64, in blocks of 128: 97 us at five,
+// 87 at six, 82 at eight; blocks of 256 threads 123)
 template <typename T, int NB>
-constexpr int BlockApplyMinBlocks() { return NB == 1 ? 12 : sizeof(T) == 8 && NB == 4 ? 4 : 8; }
+constexpr int BlockApplyMinBlocks() { return NB == 1 ? 9 : sizeof(T) == 8 && NB == 4 ? 3 : 6; }
 
-// y = B^{-1} x (or B^{-T} x). A block of 128 threads holds K whole cells, a
-// thread one cell and AP consecutive ordinates at a time (one 16-byte run of
+// y = B^{-1} x (or B^{-T} x). A block holds K whole cells, a thread one cell and AP consecutive ordinates at a time (one 16-byte run of
 // each row). The cells' shape data are staged in shared memory by cp.async
 // beside the loads of x. Bound by issue: about 230 instructions per (cell,
 // ordinate), half of them FP64, none behind a branch that splits a warp. A
 // thread per (cell, ordinate) with branches on the signs of the face terms and on
 // the pivots, its shapes gathered through L1, and this kernel, S8, FP64 / FP32:
-// 256^2 triangles 152 / 77 -> 82 / 48 us (0.46 / 0.40 of the copy bandwidth),
-// 301 x 257 quadrilaterals 108 / 50 -> 56 / 35, 48^3 hexahedra 657 / 255 -> 295 /
-// 138, 23 x 21 x 19 cubes of tetrahedra at S6 191 / 75 -> 81 / 47.
+// 256^2 triangles 153 / 77 -> 86 / 49 us (0.45 / 0.39 of the copy bandwidth),
+// 301 x 257 quadrilaterals 108 / 49 -> 58 / 36, 40^3 hexahedra 405 / 154 -> 188 /
+// 86, 20^3 cubes of tetrahedra 273 / 107 -> 118 / 56.
 template <typename T, int NB, int F, int AP, bool TRANS>
 __global__ void __launch_bounds__(kBlockThreads, BlockApplyMinBlocks<T, NB>())
    BlockApplyKernel(const DevGeom<T> g, const T *__restrict__ x, T *__restrict__ y, int K)
@@ -103,12 +106,12 @@ __global__ void __launch_bounds__(kBlockThreads, BlockApplyMinBlocks<T, NB>())
    const int A = g.A, QA = A / AP;
    const int64_t c0 = (int64_t)blockIdx.x * K;
    const int kc = (int)min((int64_t)K, g.n_cells - c0);
-   for (int e = threadIdx.x; e < kc * Rec::kUnits; e += kBlockThreads) {
+   for (int e = threadIdx.x; e < kc * Rec::kUnits; e += (int)blockDim.x) {
       const int k = e / Rec::kUnits, u = e - k * Rec::kUnits;
       CpAsync<16>(recs + k * Rec::kSize + u * Rec::kUnit, g.rec + (int64_t)g.cls[c0 + k] * kRecSize + Rec::Source(u));
    }
    bool staged = false;
-   for (int e0 = 0; e0 < kc * QA; e0 += kBlockThreads) {
+   for (int e0 = 0; e0 < kc * QA; e0 += (int)blockDim.x) {
       const int e = min(e0 + (int)threadIdx.x, kc * QA - 1);
       const int k = e / QA, a0 = (e - k * QA) * AP;
       const int64_t c = c0 + k;
@@ -169,6 +172,26 @@ __global__ void __launch_bounds__(kBlockThreads, BlockApplyMinBlocks<T, NB>())
    }
 }
 
+// The same, a thread per (cell, ordinate) that reads its cell's shape data
+// itself (LaunchBlockApply says where)
+template <typename T, int NB, int F, bool TRANS>
+__global__ void __launch_bounds__(256) BlockApplyDirectKernel(const DevGeom<T> g, const T *__restrict__ x, T *__restrict__ y)
+{
+   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+   if (tid >= g.n_cells * g.A) return;
+   const int64_t c = tid / g.A;
+   const int a = (int)(tid - c * g.A);
+   const T om[3] = {g.omega[3 * a], g.omega[3 * a + 1], g.omega[3 * a + 2]};
+   T B[NB][NB], r[NB];
+   BuildBlock<T, NB, F>(g, g.cls[c], om, g.sigma_t[c], B);
+   if constexpr (TRANS) Transpose<T, NB>(B);
+#pragma unroll
+   for (int j = 0; j < NB; j++) r[j] = x[(c * NB + j) * g.A + a];
+   const bool ok = SolveBlock<T, NB>(B, r);
+#pragma unroll
+   for (int j = 0; j < NB; j++) y[(c * NB + j) * g.A + a] = ok ? r[j] : T(0);
+}
+
 // Singular-block census (ElementBlockInverse::setup's check,
 // block_inversek.kokkos.cxx:291-296)
 template <typename T, int NB, int F>
@@ -209,20 +232,57 @@ __global__ void BlockInverseKernel(const DevGeom<T> g, T *__restrict__ inv)
       for (int j = 0; j < NB; j++) inv[(b * NB + i) * NB + j] = ok ? w[i][j] : T(0);
 }
 
+struct BlockShape {
+   int cells, threads;
+};
+
+// Whole cells of QA threads each to a block: as many as 128 threads hold, up to
+// 160 where that leaves a tenth fewer lanes idle (FP64 S16 on 256^2 DG0
+// triangles, 72 threads a cell: 174 -> 130 us); a cell of more than 160 in
+// rounds of equal length
+static BlockShape BlockApplyShape(int QA)
+{
+   const auto warps = [](int n) { return (n + 31) / 32; };
+   if (QA > kBlockThreads) {
+      const int rounds = (QA + kBlockThreads - 1) / kBlockThreads;
+      return {1, 32 * warps((QA + rounds - 1) / rounds)};
+   }
+   int K = std::max(1, 128 / QA);
+   for (int k = K + 1; k * QA <= kBlockThreads; k++)
+      if (10 * k * warps(K * QA) > 11 * K * warps(k * QA)) K = k;
+   return {K, 32 * warps(K * QA)};
+}
+
 template <typename T, int NB, int F>
 static int LaunchBlockApply(const DevGeom<T> &g, const T *x, T *y, bool trans, cudaStream_t s)
 {
-   // Ordinates per thread as one 16-byte run where they divide evenly and both
-   // vectors are 16-byte aligned; as many cells as 128 threads hold
+   // Ordinates per thread as one 16-byte run where they divide evenly, both
+   // vectors are 16-byte aligned and a cell has three runs or more: with
+   // fewer a block holds the shapes of so many cells that few fit an SM (S2,
+   // two runs, FP64: 256^2 triangles 40 us in runs and 32 one by one)
    constexpr int AV = 16 / (int)sizeof(T);
-   const bool vec = g.A % AV == 0 && (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16 == 0;
+   const bool vec = g.A % AV == 0 && g.A / AV >= 3 &&
+                    (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16 == 0;
+   // Without staging where that only delays: DG0 one by one, a division per
+   // value (256^2 triangles S16 FP64 off a 16-byte boundary: 187 us staged,
+   // 122), and DG1 triangles of four ordinates (S2), which use half of the
+   // shape data staged for them (256^2: 25 us, 19)
+   if constexpr (NB == 1 || F == 3)
+      if (!vec && (NB == 1 || g.A <= 4)) {
+         const int64_t n = g.n_cells * g.A;
+         const unsigned grid = (unsigned)((n + 255) / 256);
+         if (trans) BlockApplyDirectKernel<T, NB, F, true><<<grid, 256, 0, s>>>(g, x, y);
+         else BlockApplyDirectKernel<T, NB, F, false><<<grid, 256, 0, s>>>(g, x, y);
+         return CheckLaunch("block_apply");
+      }
    const int QA = g.A / (vec ? AV : 1);
-   const int K = std::max(1, kBlockThreads / QA);
+   const BlockShape shape = BlockApplyShape(QA);
+   const int K = shape.cells, threads = shape.threads;
    const size_t smem = (size_t)K * OwnRecord<T, NB, F>::kSize * sizeof(T);
    auto kern = vec ? (trans ? BlockApplyKernel<T, NB, F, AV, true> : BlockApplyKernel<T, NB, F, AV, false>)
                    : (trans ? BlockApplyKernel<T, NB, F, 1, true> : BlockApplyKernel<T, NB, F, 1, false>);
    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-   kern<<<(g.n_cells + K - 1) / K, kBlockThreads, smem, s>>>(g, x, y, K);
+   kern<<<(g.n_cells + K - 1) / K, threads, smem, s>>>(g, x, y, K);
    return CheckLaunch("block_apply");
 }
 
