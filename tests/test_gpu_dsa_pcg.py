@@ -60,3 +60,31 @@ def test_inner_solve_matches_numpy(case):
     v = dsa.spmv(torch.tensor(rhs, device="cuda")).cpu().numpy()
     assert np.linalg.norm(v - D @ rhs) <= 1e-13 * np.linalg.norm(D @ rhs)
     ctx.close()
+
+
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("case", ["one_block", "blocks_and_a_rest", "dg0"])
+def test_spmv_of_an_infinite_boundary_value(case, bad):
+    """A value that is not finite reaches the rows that have an entry for it,
+    and a face without a neighbour adds nothing."""
+    make, order = CASES[case]
+    rng = np.random.default_rng(4)
+    m = make(rng)
+    g, q = P.build_geometry(m, order), P.lqn(m.dim, 2)
+    st = rng.uniform(0.5, 3.0, g.n_cells)
+    ctx = T.Context(g, q)
+    keep = (torch.tensor(st, device="cuda"), torch.tensor(0.5 * st, device="cuda"))
+    ctx.set_group(*keep)
+    dsa = T.DSAPrecon(ctx)
+    dsa.set_group()
+    u = rng.standard_normal(ctx.n_nodes)
+    u[0] = u[-1] = bad  # a corner cell's first, another's last
+    with np.errstate(invalid="ignore"):
+        want = dsa.matrix() @ u
+    got = dsa.spmv(torch.tensor(u, device="cuda")).cpu().numpy()
+    assert np.isinf(want).any() or np.isnan(bad)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
+    ok = np.isfinite(want)
+    assert np.array_equal(np.sign(got[np.isinf(want)]), np.sign(want[np.isinf(want)]))
+    assert np.abs(got[ok] - want[ok]).max() <= 1e-13 * np.abs(want[ok]).max()
+    ctx.close()

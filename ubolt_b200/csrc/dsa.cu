@@ -86,22 +86,21 @@ constexpr int64_t kPcgKeepBytes = 220 * 1024;
 // A cell's matrix in shared memory, an odd number of values apart (no bank conflicts)
 __host__ __device__ constexpr int KeptStride(int F, int NB) { return (F + 1) * NB * NB | 1; }
 
-// A cell's neighbours. A face without one has zero blocks: it reads the cell
-// itself, so that no lane branches on its own
 template <int F>
 __device__ __forceinline__ void CellNeighbours(int64_t c, const int32_t *__restrict__ code, int32_t (&nbr)[F])
 {
 #pragma unroll
-   for (int f = 0; f < F; f++) {
-      const int32_t n = code[c * F + f];
-      nbr[f] = n < 0 ? (int32_t)c : n;
-   }
+   for (int f = 0; f < F; f++) nbr[f] = code[c * F + f];
 }
 
-// sum_{f, j} D(i; f, j) x(f, j) over a cell's neighbours and itself for its NB
-// rows: x(cell, j) given by `at`, element k of the cell's matrix by `val`
+// sum_{f, j} D(i; f, j) x(f, j) over cell c's neighbours and itself for its NB
+// rows: x(cell, j) given by `at`, element k of the cell's matrix by `val`. A
+// face without a neighbour has a zero block: it reads the cell itself, so that
+// no lane branches on its own, and takes zero for it (an infinite value times
+// a zero block would not be nothing)
 template <int NB, int F, typename Val, typename At>
-__device__ __forceinline__ void CellRows(const int32_t (&nbr)[F], Val val, const double (&own)[NB], At at, double (&s)[NB])
+__device__ __forceinline__ void CellRows(int64_t c, const int32_t (&nbr)[F], Val val, const double (&own)[NB], At at,
+                                         double (&s)[NB])
 {
 #pragma unroll
    for (int i = 0; i < NB; i++) s[i] = 0.0;
@@ -109,7 +108,10 @@ __device__ __forceinline__ void CellRows(const int32_t (&nbr)[F], Val val, const
    for (int f = 0; f < F; f++) {
       double x[NB];
 #pragma unroll
-      for (int j = 0; j < NB; j++) x[j] = at(nbr[f], j);
+      for (int j = 0; j < NB; j++) {
+         const double v = at(nbr[f] < 0 ? (int32_t)c : nbr[f], j);
+         x[j] = nbr[f] < 0 ? 0.0 : v;
+      }
 #pragma unroll
       for (int i = 0; i < NB; i++)
 #pragma unroll
@@ -134,7 +136,7 @@ __global__ void __launch_bounds__(128) DsaSpmvKernel(int64_t nc, const int32_t *
    for (int j = 0; j < NB; j++) own[j] = u[c * NB + j];
    int32_t nbr[F];
    CellNeighbours<F>(c, code, nbr);
-   CellRows<NB, F>(nbr, [&](int k) { return __ldg(val + (int64_t)k * nc + c); }, own,
+   CellRows<NB, F>(c, nbr, [&](int k) { return __ldg(val + (int64_t)k * nc + c); }, own,
                    [&](int32_t n, int j) { return u[(int64_t)n * NB + j]; }, s);
 #pragma unroll
    for (int i = 0; i < NB; i++) v[c * NB + i] = s[i];
@@ -347,8 +349,8 @@ __global__ void __launch_bounds__(kPcgThreads, kPcgBlocksPerSm) DsaPcgKernel(con
          } else {
             if constexpr (!OWN) CellNeighbours<F>(c, a.code, nbr);
             auto at = [&](int32_t n, int j) { return direction((int64_t)n * NB + j); };
-            if constexpr (KEEP) CellRows<NB, F>(nbr, [&](int k) { return mine[k]; }, p, at, q);
-            else CellRows<NB, F>(nbr, [&](int k) { return __ldg(a.val + (int64_t)k * a.n + c); }, p, at, q);
+            if constexpr (KEEP) CellRows<NB, F>(c, nbr, [&](int k) { return mine[k]; }, p, at, q);
+            else CellRows<NB, F>(c, nbr, [&](int k) { return __ldg(a.val + (int64_t)k * a.n + c); }, p, at, q);
          }
 #pragma unroll
          for (int i = 0; i < NB; i++) {
