@@ -88,3 +88,26 @@ def test_spmv_of_an_infinite_boundary_value(case, bad):
     assert np.array_equal(np.sign(got[np.isinf(want)]), np.sign(want[np.isinf(want)]))
     assert np.abs(got[ok] - want[ok]).max() <= 1e-13 * np.abs(want[ok]).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("name, make", [
+    ("tri", lambda r: P.box_tris(160, 153, jitter=0.2, rng=r)), ("tri_more", lambda r: P.box_tris(161, 154, jitter=0.2, rng=r)),
+    ("quad_more", lambda r: P.box_quads(231, 221, jitter=0.2, rng=r)),
+    ("tet_more", lambda r: P.box_tets(21, 20, 20, jitter=0.2, rng=r)), ("hex_more", lambda r: P.box_hexes(38, 37, 36))])
+def test_spmv_by_rows_and_by_cells(name, make):
+    """Either side of the mesh size (49152 cells) at which the multiply changes from a
+    thread per row to a thread per cell."""
+    rng = np.random.default_rng(6)
+    g, q = P.build_geometry(make(rng), 1), P.lqn(3 if name[0] in "h" or name[:3] == "tet" else 2, 2)
+    assert (g.n_cells > 49152) == name.endswith("_more")
+    st = rng.uniform(0.5, 3.0, g.n_cells)
+    ctx = T.Context(g, q)
+    keep = (torch.tensor(st, device="cuda"), torch.tensor(0.5 * st, device="cuda"))
+    ctx.set_group(*keep)
+    dsa = T.DSAPrecon(ctx)
+    dsa.set_group()
+    u = rng.standard_normal(ctx.n_nodes)
+    want = dsa.matrix() @ u
+    got = dsa.spmv(torch.tensor(u, device="cuda")).cpu().numpy()
+    assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
+    ctx.close()

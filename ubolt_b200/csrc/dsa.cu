@@ -83,6 +83,8 @@ namespace ubolt {
 // shared memory a block may hold of the matrix
 constexpr int kPcgThreads = 512, kPcgBlocksPerSm = 1;
 constexpr int64_t kPcgKeepBytes = 220 * 1024;
+// Most cells of a multiply by rows (see DsaSpmvLaunch)
+constexpr int64_t kSpmvRowCells = 49152;
 // A cell's matrix in shared memory, an odd number of values apart (no bank conflicts)
 __host__ __device__ constexpr int KeptStride(int F, int NB) { return (F + 1) * NB * NB | 1; }
 
@@ -142,6 +144,36 @@ __global__ void __launch_bounds__(128) DsaSpmvKernel(int64_t nc, const int32_t *
    for (int i = 0; i < NB; i++) v[c * NB + i] = s[i];
 }
 
+// The same with a thread per row (grid.y: the row within the cell), all of whose
+// loads are in flight at once
+template <int NB, int F>
+__global__ void __launch_bounds__(128) DsaSpmvRowKernel(int64_t nc, const int32_t *__restrict__ code,
+                                                        const double *__restrict__ val, const double *__restrict__ u,
+                                                        double *__restrict__ v)
+{
+   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+   const int i = blockIdx.y;
+   if (c >= nc) return;
+   int32_t nbr[F];
+   CellNeighbours<F>(c, code, nbr);
+   double d[F + 1][NB], x[F + 1][NB];
+#pragma unroll
+   for (int f = 0; f <= F; f++)
+#pragma unroll
+      for (int j = 0; j < NB; j++) {
+         const int32_t n = f < F ? nbr[f < F ? f : 0] : (int32_t)c;
+         d[f][j] = __ldg(val + (int64_t)((f * NB + i) * NB + j) * nc + c);
+         const double xv = u[(n < 0 ? c : (int64_t)n) * NB + j];
+         x[f][j] = n < 0 ? 0.0 : xv;
+      }
+   double s = 0.0;
+#pragma unroll
+   for (int f = 0; f <= F; f++)
+#pragma unroll
+      for (int j = 0; j < NB; j++) s += d[f][j] * x[f][j];
+   v[c * NB + i] = s;
+}
+
 // v = D u over CSR rows (the CG-SUPG vertices), one thread per row
 __global__ void DsaCsrSpmvKernel(int64_t n_nodes, const int64_t *__restrict__ rp, const int32_t *__restrict__ col,
                                  const double *__restrict__ val, const double *__restrict__ u, double *__restrict__ v)
@@ -160,8 +192,15 @@ static int DsaSpmvLaunch(const ubolt_ctx *ctx, const ubolt_dsa *ds, const double
       DsaCsrSpmvKernel<<<(ds->n_nodes + 127) / 128, 128, 0, s>>>(ds->n_nodes, ds->d_rp, ds->d_col, ds->val, u, v);
       return CheckLaunch("dsa_spmv");
    }
+   // A small mesh takes a round trip to memory or two: rows side by side. A large
+   // one is bound by the matrix, and a thread per cell reads u once (rows and
+   // cells, us, after other work: 4080 hexahedra 12 and 18, 48 k tetrahedra 15 and
+   // 18; again and again: 64 k hexahedra 12.7 and 8.5, 2 M triangles 155 and 103)
+   const bool rows = ds->nb > 1 && ds->nc <= kSpmvRowCells;
+   const unsigned grid = (unsigned)((ds->nc + 127) / 128);
    UBOLT_DISPATCH(ds->nb, ds->F, {
-      DsaSpmvKernel<NB_, F_><<<(ds->nc + 127) / 128, 128, 0, s>>>(ds->nc, ctx->g64.code, ds->val, u, v);
+      if (rows) DsaSpmvRowKernel<NB_, F_><<<dim3(grid, NB_), 128, 0, s>>>(ds->nc, ctx->g64.code, ds->val, u, v);
+      else DsaSpmvKernel<NB_, F_><<<grid, 128, 0, s>>>(ds->nc, ctx->g64.code, ds->val, u, v);
       return CheckLaunch("dsa_spmv");
    });
    return SetError(UBOLT_ERR_STATE, "no DSA kernel for this shape");
