@@ -62,7 +62,7 @@ struct ubolt_dsa {
    std::vector<double> area, nrm, dist, volume, fown, fup, bgrad, nbgrad, half_range;
    std::vector<int64_t> nbr;
    std::vector<int32_t> bc;
-   std::vector<double> h_val, h_jinv;
+   std::vector<double> h_val, h_jinv;  // cell by cell: [nc][F+1][nb][nb], [nc][nb][nb] (CG: as on the device)
    // CG-SUPG: the vertex CSR, and per (element, li, j) its entry
    bool cg = false;
    std::vector<int64_t> rp, entry;
@@ -73,6 +73,8 @@ struct ubolt_dsa {
    // Device
    double *val = nullptr, *jinv = nullptr;          // [F+1][nb][nb][nc], [nb][nb][nc] (CG: [nnz], [n_nodes])
    double *rhs = nullptr, *u = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr;
+   double *stage = nullptr;  // an upload's cells as the host has them (DG)
+   int64_t stage_doubles = 0;
    double *slots = nullptr;  // the grid sums' counter (in two words' place), then two slots per block
 };
 
@@ -612,19 +614,13 @@ static int Assemble(ubolt_dsa *ds, const double *st, const double *ss)
    const uint8_t *masked = ds->h_mask.data(), *is_void = ds->h_void.data();
 #pragma omp parallel for schedule(static)
    for (int64_t c = 0; c < nc; c++) {
-      double blk[(kMaxFaces + 1) * kMaxNb * kMaxNb] = {0.0}, inv[kMaxNb * kMaxNb];
-      double *own = blk + F * bs;
+      double *blk = &ds->h_val[c * (F + 1) * bs], *own = blk + F * bs;
+      std::fill(blk, blk + (F + 1) * bs, 0.0);
       const double vol = ds->volume[c];
-      // Into the element-major stores
-      auto store = [&]() {
-         InvertSmall(nb, own, inv);
-         for (size_t k = 0; k < (F + 1) * bs; k++) ds->h_val[k * nc + c] = blk[k];
-         for (size_t k = 0; k < bs; k++) ds->h_jinv[k * nc + c] = inv[k];
-      };
       if (masked[c]) {
          // A masked void: V times the identity, every coupling zero
          for (int i = 0; i < nb; i++) own[i * nb + i] = vol;
-         store();
+         InvertSmall(nb, own, &ds->h_jinv[c * bs]);
          continue;
       }
       const double d_c = dcell[c];
@@ -706,9 +702,45 @@ static int Assemble(ubolt_dsa *ds, const double *st, const double *ss)
             }
          }
       }
-      store();
+      InvertSmall(nb, own, &ds->h_jinv[c * bs]);
    }
    return UBOLT_OK;
+}
+
+// in[n][per], cell by cell, to out[k nc + c] for k < per, through shared memory:
+// runs of 32 cells on the way out. Written so by the host, a value every nc
+// words, the assembly of a group took several times as long as cell by cell
+// where nc is a multiple of some thousands (32768 tetrahedra, the stores alone:
+// 3.2 and 0.3 ms)
+constexpr int kElementCells = 32;
+__global__ void __launch_bounds__(256) DsaElementMajorKernel(const double *__restrict__ in, int64_t n, int per, int64_t nc,
+                                                             double *__restrict__ out)
+{
+   __shared__ double tile[kElementCells * ((kMaxFaces + 1) * kMaxNb * kMaxNb + 1)];
+   const int64_t c0 = (int64_t)blockIdx.x * kElementCells;
+   const int cells = (int)min((int64_t)kElementCells, n - c0);
+   for (int e = threadIdx.x; e < cells * per; e += 256) {
+      const int c = e / per, k = e - c * per;
+      tile[c * (per + 1) + k] = in[c0 * per + e];
+   }
+   __syncthreads();
+   const int lane = threadIdx.x & 31;
+   if (lane < cells)
+      for (int k = threadIdx.x >> 5; k < per; k += 8) out[(int64_t)k * nc + c0 + lane] = tile[lane * (per + 1) + k];
+}
+
+// A host array of nc cells, `per` values each, to the device element by element
+static void UploadElementMajor(const ubolt_dsa *ds, const std::vector<double> &host, double *out, cudaStream_t s)
+{
+   const int per = (int)(host.size() / ds->nc);
+   const int64_t at_once = ds->stage_doubles / per;
+   for (int64_t c0 = 0; c0 < ds->nc; c0 += at_once) {
+      const int64_t n = std::min(at_once, ds->nc - c0);
+      cudaMemcpyAsync(ds->stage, host.data() + c0 * per, (size_t)(n * per) * sizeof(double), cudaMemcpyHostToDevice, s);
+      DsaElementMajorKernel<<<(unsigned)((n + kElementCells - 1) / kElementCells), 256, 0, s>>>(ds->stage, n, per, ds->nc,
+                                                                                              out + c0);
+      CountLaunch();
+   }
 }
 
 // The CG-SUPG vertex operator for one group (DSACG::assemble,
@@ -819,7 +851,7 @@ void UboltDsaFree(ubolt_ctx *ctx)
    ubolt_dsa *ds = ctx->dsa;
    if (!ds) return;
    for (void *p : {(void *)ds->val, (void *)ds->jinv, (void *)ds->rhs, (void *)ds->u, (void *)ds->r, (void *)ds->z,
-                   (void *)ds->p, (void *)ds->q, (void *)ds->slots, (void *)ds->mask, (void *)ds->d_rp,
+                   (void *)ds->p, (void *)ds->q, (void *)ds->slots, (void *)ds->stage, (void *)ds->mask, (void *)ds->d_rp,
                    (void *)ds->d_col})
       if (p) cudaFree(p);
    delete ds;
@@ -855,7 +887,10 @@ static int AllocDsa(ubolt_dsa *ds, size_t n_val, size_t n_jinv)
       return UBOLT_OK;
    };
    const size_t nn = (size_t)ds->n_nodes;
+   // (an upload in parts: at most 32 MB, at least one cell)
+   ds->stage_doubles = ds->cg ? 0 : std::max<int64_t>(std::min<int64_t>((int64_t)n_val, 4 << 20), 128);
    int rc = 0;
+   if (ds->stage_doubles && (rc = alloc(&ds->stage, (size_t)ds->stage_doubles))) return rc;
    if ((rc = alloc(&ds->val, n_val)) || (rc = alloc(&ds->jinv, n_jinv)) || (rc = alloc(&ds->rhs, nn)) ||
        (rc = alloc(&ds->u, nn)) || (rc = alloc(&ds->r, nn)) || (rc = alloc(&ds->z, nn)) || (rc = alloc(&ds->p, nn)) ||
        (rc = alloc(&ds->q, nn)) || (rc = alloc(&ds->slots, 2 + 2 * PcgMostBlocks(nn))))
@@ -1049,8 +1084,13 @@ extern "C" int ubolt_dsa_set_group(ubolt_ctx *ctx, void *stream)
    cudaMemcpyAsync(ss.data(), ctx->g64.sigma_s, ds->nc * 8, cudaMemcpyDeviceToHost, s);
    if ((rc = CudaCheck(cudaStreamSynchronize(s), "dsa_set_group"))) return rc;
    if ((rc = ds->cg ? AssembleCg(ctx, ds, st.data(), ss.data()) : Assemble(ds, st.data(), ss.data()))) return rc;
-   cudaMemcpyAsync(ds->val, ds->h_val.data(), ds->h_val.size() * 8, cudaMemcpyHostToDevice, s);
-   cudaMemcpyAsync(ds->jinv, ds->h_jinv.data(), ds->h_jinv.size() * 8, cudaMemcpyHostToDevice, s);
+   if (ds->cg) {
+      cudaMemcpyAsync(ds->val, ds->h_val.data(), ds->h_val.size() * 8, cudaMemcpyHostToDevice, s);
+      cudaMemcpyAsync(ds->jinv, ds->h_jinv.data(), ds->h_jinv.size() * 8, cudaMemcpyHostToDevice, s);
+   } else {
+      UploadElementMajor(ds, ds->h_val, ds->val, s);
+      UploadElementMajor(ds, ds->h_jinv, ds->jinv, s);
+   }
    if (ds->mask) cudaMemcpyAsync(ds->mask, ds->h_mask.data(), ds->nc, cudaMemcpyHostToDevice, s);
    if ((rc = CudaCheck(cudaStreamSynchronize(s), "dsa upload"))) return rc;
    ds->assembled = true;
@@ -1117,10 +1157,7 @@ extern "C" int ubolt_dsa_matrix(ubolt_ctx *ctx, double *blocks)
    if (rc || (rc = CheckDsa(ctx))) return rc;
    if (!blocks) return SetError(UBOLT_ERR_ARG, "dsa_matrix: NULL output");
    if (ctx->dsa->cg) return SetError(UBOLT_ERR_STATE, "dsa_matrix: the CG-SUPG operator is CSR, read it by ubolt_dsa_spmv");
-   const ubolt_dsa *ds = ctx->dsa;
-   const size_t per = (size_t)(ds->F + 1) * ds->nb * ds->nb;
-   for (int64_t c = 0; c < ds->nc; c++)
-      for (size_t k = 0; k < per; k++) blocks[c * per + k] = ds->h_val[k * ds->nc + c];
+   std::copy(ctx->dsa->h_val.begin(), ctx->dsa->h_val.end(), blocks);
    return UBOLT_OK;
 }
 
