@@ -111,3 +111,41 @@ def test_spmv_by_rows_and_by_cells(name, make):
     got = dsa.spmv(torch.tensor(u, device="cuda")).cpu().numpy()
     assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("nx, ny", [(40, 31), (300, 280), (400, 390)])
+def test_vertex_inner_solve_matches_numpy(nx, ny):
+    """The CG-SUPG vertices' inner solve: one per thread, and more than the
+    threads of one block per SM and of two. Against the oracle's matrix."""
+    import cg as OC
+    rng = np.random.default_rng(8)
+    m = P.box_quads(nx, ny, jitter=0.2, rng=rng)
+    g, q = P.build_cg_geometry(m), P.lqn(2, 2)
+    st = rng.uniform(0.5, 3.0, g.n_elements)
+    ss = st * rng.uniform(0.3, 0.9, g.n_elements)
+    ctx = T.Context(g, q)
+    keep = (torch.tensor(st, device="cuda"), torch.tensor(ss, device="cuda"))
+    ctx.set_group(*keep)
+    its = 6
+    dsa = T.DSAPrecon(ctx, inner_iterations=its)
+    dsa.set_group()
+    ref = OC.Problem(m, q, st, ss)
+    D = ref.dsa_matrix()[0]
+    x = rng.standard_normal(ctx.n_rows)
+    rhs = ref.dsa_restrict(x)
+    jac = 1.0 / D.diagonal()
+    u, r = np.zeros_like(rhs), rhs.copy()
+    z = jac * r
+    p, rho = z.copy(), r @ z
+    for _ in range(its):
+        s = D @ p
+        alpha = rho / (p @ s)
+        u, r = u + alpha * p, r - alpha * s
+        z = jac * r
+        new = r @ z
+        p, rho = z + new / rho * p, new
+    want = ref.dsa_prolong(u)
+    y = dsa.apply(torch.tensor(x, device="cuda")).cpu().numpy()
+    # Six iterations amplify rounding by far less than 1e5
+    assert np.linalg.norm(y - want) <= 1e-11 * np.linalg.norm(want)
+    ctx.close()

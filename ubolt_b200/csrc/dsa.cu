@@ -81,9 +81,14 @@ struct ubolt_dsa {
 namespace ubolt {
 
 // The PCG's blocks: one of 512 threads per SM (at two of 384 the kernel
-// spilled, and a spill is a trip to L2 here, as every grid sum empties L1), and the
-// shared memory a block may hold of the matrix
-constexpr int kPcgThreads = 512, kPcgBlocksPerSm = 1;
+// spilled, and a spill is a trip to L2 here, as every grid sum empties L1), two
+// for vertices that outnumber the threads of one: their rows are short, scattered
+// reads, which want warps in flight (an apply on 100^3 hexahedra, 1.03 M vertices:
+// 9.3 ms with one, 5.0 with two, 6.7 with three, 4.9 launch by launch; 1200^2
+// quadrilaterals 4.3, 2.8, 2.7, 3.3). And the shared memory a block may hold of
+// the matrix
+constexpr int kPcgThreads = 512;
+constexpr int PcgBlocksPerSm(bool csr, bool own) { return csr && !own ? 2 : 1; }
 constexpr int64_t kPcgKeepBytes = 220 * 1024;
 // Most cells of a multiply by rows (see DsaSpmvLaunch)
 constexpr int64_t kSpmvRowCells = 49152;
@@ -320,7 +325,7 @@ __device__ __forceinline__ bool GridSum(double d, const DsaPcgArgs &a, unsigned 
 // cells than threads) 1266 -> 731, 32^3 hexahedra 905 -> 426, 16^3 cubes of
 // tetrahedra 832 -> 385, 24^2 triangles 667 -> 199.
 template <int NB, int F, bool CSR, bool OWN, bool KEEP>
-__global__ void __launch_bounds__(kPcgThreads, kPcgBlocksPerSm) DsaPcgKernel(const DsaPcgArgs a)
+__global__ void __launch_bounds__(kPcgThreads, PcgBlocksPerSm(CSR, OWN)) DsaPcgKernel(const DsaPcgArgs a)
 {
    extern __shared__ double kept[];  // KEEP: [cells of a block][KeptStride], a thread's run at fixed offsets
    double *mine = kept + threadIdx.x * KeptStride(F, NB);
@@ -443,16 +448,17 @@ static int LaunchPcg(const DsaPcgArgs &args, cudaStream_t s)
    int dev = 0, sms = 0;
    cudaGetDevice(&dev);
    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-   const int64_t most = std::min<int64_t>((int64_t)sms * kPcgBlocksPerSm, 1024);
+   int64_t most = std::min<int64_t>((int64_t)sms * PcgBlocksPerSm(CSR, true), 1024);
    // As many cells per block as its threads, or as its shared memory holds
    // where that still covers every cell with the blocks that run at once
    constexpr int64_t kCellBytes = CSR ? 1 << 30 : KeptStride(F, NB) * (int64_t)sizeof(double);
    const int64_t fit = std::min<int64_t>(kPcgThreads, kPcgKeepBytes / kCellBytes);
    const bool keep = fit > 0 && args.n <= fit * most;
    const int64_t want = keep ? (args.n + fit - 1) / fit : (args.n + kPcgThreads - 1) / kPcgThreads;
+   const bool own = want <= most;
+   if (!own) most = std::min<int64_t>((int64_t)sms * PcgBlocksPerSm(CSR, false), 1024);
    const int grid = (int)std::max<int64_t>(1, std::min(most, want));
    const int64_t per = (args.n + grid - 1) / grid;
-   const bool own = per <= kPcgThreads;
    auto kern = keep ? DsaPcgKernel<NB, F, CSR, true, !CSR>
                : own ? DsaPcgKernel<NB, F, CSR, true, false> : DsaPcgKernel<NB, F, CSR, false, false>;
    const size_t smem = keep ? (size_t)(per * kCellBytes) : 0;
