@@ -87,6 +87,7 @@ __device__ __forceinline__ T BoundaryTerms(const CgDev<T> &d, int64_t i, int a, 
 }
 
 constexpr int kCgThreads = 128;
+constexpr int64_t kSms = 148;
 // Shared memory of one chunk of star entries
 constexpr int kCgChunkBytes = 48 * 1024;
 
@@ -234,6 +235,44 @@ __global__ void __launch_bounds__(kCgThreads, CgMinBlocks<T, DIM, AP>()) CgApply
          StoreRun<T, AP>(y + i * A + a0, out);
       }
    }
+}
+
+// The same, a thread per row that walks its star itself (LaunchCgApply says where)
+template <typename T, int DIM, int NV, bool SCATTER>
+__global__ void __launch_bounds__(256) CgApplyDirectKernel(const CgDev<T> d, const T *__restrict__ x,
+                                                           const T *__restrict__ phi, T *__restrict__ y)
+{
+   constexpr int P = CgRecordSize(DIM);
+   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+   if (r >= d.n_rows) return;
+   const int64_t i = r / d.A;
+   const int a = (int)(r - i * d.A);
+   T om[DIM];
+#pragma unroll
+   for (int c = 0; c < DIM; c++) om[c] = d.omega[3 * a + c];
+   T acc = T(0), sacc = T(0);
+   const int s1 = d.star_off[i + 1];
+   for (int s = d.star_off[i]; s < s1; s++) {
+      const int e = d.star_elem[s];
+      const T st = d.sigma_t[e];
+      const T tau = d.tau[(int64_t)e * d.A + a];
+      const T *rec = d.rec + (int64_t)s * NV * P;
+      const int32_t *col = d.cols + (int64_t)s * NV;
+      T srow = T(0);
+#pragma unroll
+      for (int j = 0; j < NV; j++) {
+         const T *q = rec + j * P;
+         const T w = q[0] + tau * DotD<T, DIM>(om, q + 1 + DIM);
+         const T coef = DotD<T, DIM>(om, q + 1) + tau * OmegaKOmega<T, DIM>(q + 1 + 2 * DIM, om) + st * w;
+         const int64_t v = col[j];
+         acc += coef * x[v * d.A + a];
+         if constexpr (SCATTER) srow += w * phi[v];
+      }
+      if constexpr (SCATTER) sacc += d.sigma_s[e] * srow;
+   }
+   T out = acc;
+   if constexpr (SCATTER) out -= sacc * d.inv_sum_weights;
+   y[r] = out * d.inv_m[i] + BoundaryTerms<T, DIM>(d, i, a, om, x);
 }
 
 // The diagonal of L (the assembled term's diagonal slot, SUPGTermCG::
@@ -407,13 +446,30 @@ static int LaunchCgApply(const CgDev<T> &d, int max_star, const T *x, const T *p
    // As many vertices per block as 128 threads hold and as their star entries
    // fit in one chunk (few ordinates on hexahedra: 8 entries of 1 KB a vertex).
    // Ordinates per thread as one 16-byte run where they divide evenly and both
-   // vectors are 16-byte aligned, unless that leaves a block few threads
-   // (20^3 hexahedra S2, FP64: 74 us with runs in chunks against 43)
+   // vectors are 16-byte aligned, unless that leaves a block few threads: under
+   // 64 (20^3 hexahedra S2, FP64: 74 us with runs in chunks against 43), or fewer
+   // by a third than one by one where the chunk limits the vertices (301 x 257
+   // quadrilaterals S2 FP32: 40 us with runs, 31 without), or a grid of fewer than two
+   // blocks per SM, which waits for one thread's walk (31 x 27 triangles S4 FP32: 16 and 11)
    constexpr int AV = 16 / (int)sizeof(T);
    constexpr int kEntry = CgEntryBytes<T, DIM, NV>(), kMost = kCgChunkBytes / kEntry;
    const int fit = std::max(1, kMost / max_star);
+   const auto block = [&](int q) { return std::max(1, std::min(fit, kCgThreads / q)) * q; };
    const bool aligned = d.A % AV == 0 && (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16 == 0;
-   const bool vec = aligned && (int64_t)fit * (d.A / AV) >= kCgThreads / 2;
+   const int runs = d.A / AV;
+   const bool vec = aligned && fit * runs >= kCgThreads / 2 && (fit * runs >= kCgThreads || 2 * block(d.A) < 3 * block(runs)) &&
+                    (d.n_vertices * runs >= 2 * kSms * kCgThreads || d.A > kCgThreads);
+   // Eight ordinates or fewer (S2) in FP64 on a large mesh: blocks that the chunk
+   // leaves under 128 threads are too few warps to stream the records with. A
+   // thread per row (staged and so, us: 512^2 triangles 218 and 176, 40^3 cubes of
+   // tetrahedra 562 and 444, 40^3 hexahedra 290 and 274; 12^3 cubes of
+   // tetrahedra 23 and 51)
+   if (sizeof(T) == 8 && d.A <= 8 && fit * d.A < kCgThreads && d.n_rows >= 96 * 1024) {
+      const unsigned grid = (unsigned)((d.n_rows + 255) / 256);
+      if (scatter) CgApplyDirectKernel<T, DIM, NV, true><<<grid, 256, 0, s>>>(d, x, phi, y);
+      else CgApplyDirectKernel<T, DIM, NV, false><<<grid, 256, 0, s>>>(d, x, phi, y);
+      return CheckLaunch("cg apply");
+   }
    const int QA = d.A / (vec ? AV : 1);
    const int K = std::max(1, std::min(fit, kCgThreads / QA));
    const int E = std::min(K * max_star, kMost);
