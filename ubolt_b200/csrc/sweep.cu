@@ -58,6 +58,9 @@ constexpr int kSweepWarpsPerSm = 32;
 constexpr size_t kViaBytes = (size_t)8 << 20;
 constexpr uint32_t kCopyTries = 1u << 22;  // bounded wait for a task's bulk copy
 
+// Few cell-ordinates fill the device with tasks of either size
+constexpr int64_t kFewCellOrdinates = (int64_t)1 << 20;
+
 // The default patch, in cells. Larger patches make fewer and longer tasks
 // with fewer waits between them, but their couplings take the shared memory of
 // resident warps, and a task starts as late as its latest ghost. Measured per
@@ -78,8 +81,7 @@ static int DefaultPatch(const ubolt_ctx *ctx)
    const bool tets = ctx->dim == 3 && ctx->F == 4;
    if (ctx->nb == 1) return ctx->dim == 2 ? 256 : tets ? 192 : 128;
    if (ctx->dim == 3) return tets ? 48 : 64;
-   // Few cell-ordinates fill the device with tasks of either size
-   return ctx->n_cells * (int64_t)ctx->A <= (int64_t)1 << 20 ? 128 : 64;
+   return ctx->n_cells * (int64_t)ctx->A <= kFewCellOrdinates ? 128 : 64;
 }
 
 namespace ubolt {
@@ -346,17 +348,20 @@ struct SweepSlice {
 // are laid out in shared memory and written 32 positions at a time.
 // A block takes a patch: its cells' class records are staged in shared memory
 // once (STAGED, where they fit) and read by the tasks of every ordinate, a warp
-// per task. Read by a lane per position straight from global memory, every
-// load touched 32 lines, which bound the kernel (and the factors built in the
-// sweep itself). A group's factors, FP64 / FP32, a warp per task from global
-// memory and this way: 256^2 triangles S8 733 / 424 -> 448 / 300 us, 20^3 cubes
-// of tetrahedra 2095 / 1348 -> 1044 / 555, 40^3 hexahedra 2272 / 2041 -> 969 /
-// 477; a few hundred thousand cell-ordinates, where a patch's blocks are few,
-// 59 / 37 -> 75 / 41 (101 x 77 triangles S6).
+// per task or, where that leaves warps without one, per 32 positions of a task.
+// Read by a lane per position straight from global memory, every load touched 32
+// lines, which bound the kernel (and the factors built in the sweep itself). A
+// group's factors, FP64 / FP32, a warp per task from global memory and this way:
+// 256^2 triangles S8 724 / 415 -> 428 / 285 us, 20^3 cubes of tetrahedra 2088 /
+// 1339 -> 1027 / 542, 40^3 hexahedra 2263 / 2033 -> 946 / 483, 125 hexahedra S8
+// 10 / 10 -> 13 / 8. Slower on 2D meshes of a few hundred thousand cell-ordinates
+// in FP64, whose larger patches are few blocks: 101 x 77 triangles S6 50 / 31 ->
+// 60 / 35, 150^2 S4 71 / 41 -> 88 / 46; without staging there 65, a warp per 32
+// positions 90, patches of 64 cells less, but a sweep takes 5 to 10 us longer then.
 template <typename T, int NB, int F, bool STAGED>
 __global__ void __launch_bounds__(256, sizeof(T) == 8 && NB == 4 ? 1 : 2) FactorKernel(const DevGeom<T> g, const SweepDev s, T *__restrict__ fac,
                                                     const int32_t *__restrict__ patch_ptr,
-                                                    const int32_t *__restrict__ patch_task)
+                                                    const int32_t *__restrict__ patch_task, int chunks)
 {
    constexpr int RS = RecordLayout(NB, F, (int)sizeof(T)).size;
    constexpr int RP = RecordStride(RS, (int)sizeof(T));
@@ -372,21 +377,32 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 && NB == 4 ? 1 : 2) Factor
    if constexpr (STAGED) {
       constexpr int UN = RS * (int)sizeof(T) / 16;
       const int nc = (int)min((int64_t)s.P, g.n_cells - base);
-      for (int e = threadIdx.x; e < nc * UN; e += blockDim.x) {
-         const int k = e / UN, u = e - k * UN;
-         CpAsync<16>(recs + k * RP + u * (16 / (int)sizeof(T)),
-                     g.rec + (int64_t)g.cls[base + k] * RS + u * (16 / (int)sizeof(T)));
+      // A warp per record, the class ids of four read at once (a lane per 16-byte
+      // unit, each behind a class id of its own, took 10 us before the first task)
+      for (int k0 = warp; k0 < nc; k0 += 4 * n_warps) {
+         int32_t cl[4];
+#pragma unroll
+         for (int m = 0; m < 4; m++) cl[m] = g.cls[base + min(k0 + m * n_warps, nc - 1)];
+#pragma unroll
+         for (int m = 0; m < 4; m++) {
+            const int k = k0 + m * n_warps;
+            if (k < nc)
+               for (int u = lane; u < UN; u += 32)
+                  CpAsync<16>(recs + k * RP + u * (16 / (int)sizeof(T)),
+                              g.rec + (int64_t)cl[m] * RS + u * (16 / (int)sizeof(T)));
+         }
       }
       CpAsyncWaitAll();
       __syncthreads();
    }
-   for (int32_t x = patch_ptr[blockIdx.x] + warp + n_warps * (int)blockIdx.y; x < patch_ptr[blockIdx.x + 1];
-        x += n_warps * (int)gridDim.y) {
-      const Task tk = LoadTask(s.task + patch_task[x]);
+   // A warp's unit of work: a task, or every `chunks`th 32 positions of one
+   const int x0 = patch_ptr[blockIdx.x], n_units = (patch_ptr[blockIdx.x + 1] - x0) * chunks;
+   for (int x = warp + n_warps * (int)blockIdx.y; x < n_units; x += n_warps * (int)gridDim.y) {
+      const Task tk = LoadTask(s.task + patch_task[x0 + x / chunks]);
       const int ncell = tk.ncell(), a = tk.ordinate;
       const T om[3] = {g.omega[3 * a], g.omega[3 * a + 1], g.omega[3 * a + 2]};
       T *ft = fac + (size_t)tk.off * R;
-      for (int i0 = 0; i0 < ncell; i0 += 32) {
+      for (int i0 = 32 * (x % chunks); i0 < ncell; i0 += 32 * chunks) {
          // A lane past the end repeats the last position
          const int i = min(i0 + lane, ncell - 1);
          const int local = s.sched[(tk.off + i) * SchedWords(F)];
@@ -1112,11 +1128,12 @@ static T *EnsureFactors(ubolt_ctx *ctx, cudaStream_t st)
       pl->fac_epoch[which] = ctx->group_epoch;
       return static_cast<T *>(pl->fac[which]);
    }
-   int smem_max = 48 * 1024, dev = 0;
+   int smem_max = 48 * 1024, n_sm = 1, dev = 0;
    cudaGetDevice(&dev);
+   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
    cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-   // Eight warps per patch, four where the patches are few; its class
-   // records in shared memory where they fit beside the warps' staging
+   // Eight warps per patch, its class records in shared memory where they fit
+   // beside the warps' staging
    const int warps = 8;
    const size_t stage = (size_t)warps * 32 * LaneStride(pl->slots * NB * NB, (int)sizeof(T)) * sizeof(T);
    const size_t recs = (size_t)pl->P * RecordStride(RecordLayout(NB, F, (int)sizeof(T)).size, (int)sizeof(T)) * sizeof(T);
@@ -1124,10 +1141,15 @@ static T *EnsureFactors(ubolt_ctx *ctx, cudaStream_t st)
    const size_t smem = (staged ? recs : 0) + stage;
    auto kern = staged ? FactorKernel<T, NB, F, true> : FactorKernel<T, NB, F, false>;
    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-   // Large patches make few blocks: then several share a patch's tasks
-   const int parts = std::max(1, std::min((148 * 8 + pl->n_patches - 1) / pl->n_patches, (ctx->A + warps - 1) / warps));
+   // Large patches make few blocks: then several share a patch's tasks. Where all
+   // tasks' pieces of 32 positions are one for a warp at most, a warp takes a piece
+   // (64^2 DG0 quadrilaterals S4 18 -> 8 us, 16 x 15 x 17 hexahedra S2 20 -> 14; with
+   // more, 101 x 77 triangles S6 60 and 90: every block stages its patch's records)
+   const int most_chunks = (pl->P + 31) / 32;
+   const int chunks = !staged || pl->n_tasks * most_chunks <= (int64_t)n_sm * 16 ? most_chunks : 1;
+   const int parts = std::max(1, std::min((n_sm * 8 + pl->n_patches - 1) / pl->n_patches, (ctx->A * chunks + warps - 1) / warps));
    kern<<<dim3(pl->n_patches, parts), 32 * warps, smem, st>>>(ctx->geom<T>(), DevPlan(pl), static_cast<T *>(pl->fac[which]),
-                                                 pl->patch_ptr, pl->patch_task);
+                                                 pl->patch_ptr, pl->patch_task, chunks);
    if (CheckLaunch("sweep factors")) return nullptr;
    pl->fac_epoch[which] = ctx->group_epoch;
    return static_cast<T *>(pl->fac[which]);
