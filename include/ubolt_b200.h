@@ -338,8 +338,10 @@ typedef struct {
  * streamed in by bulk copies - meshes whose every ordinate's upwind graph is
  * acyclic (2D, hexahedra), with a reserved factor store, no wait on another
  * block. One block per ordinate leaves most SMs idle and pays for every
- * scattered psi word on one SM; TASKS measured faster at every size, and AUTO
- * is TASKS. */
+ * scattered psi word on one SM: AUTO takes WAVE only on small DG0 meshes of
+ * hexahedra (at most 4096 cells and 2^17 cell-ordinates), where it measured
+ * faster, and TASKS otherwise - there too for what WAVE does not do (psi
+ * ordinate-major), its factors then formed as it goes. */
 enum { UBOLT_SWEEP_AUTO = 0, UBOLT_SWEEP_TASKS = 1, UBOLT_SWEEP_WAVE = 2 };
 
 /* Build the sweep plan: patches of patch_size consecutive cells (0 picks

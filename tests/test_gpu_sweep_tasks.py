@@ -76,3 +76,52 @@ def test_task_sweep_of_nan_ends():
         assert bool(torch.isnan(sw.apply(ones)).all())
         assert sw.status()["timeouts"] == 0
     ctx.close()
+
+
+@pytest.mark.parametrize("n, order, sn, wave", [
+    ((10, 9, 11), 0, 4, True), ((16, 16, 16), 0, 2, True), ((17, 16, 16), 0, 2, False), ((10, 9, 11), 1, 4, False),
+    ((16, 16, 16), 0, 6, False)])
+def test_automatic_kernel(n, order, sn, wave):
+    """Small DG0 boxes of hexahedra take the wave kernel, up to 4096 cells and
+    2^17 cell-ordinates; ordinate-major output runs there too, and a choice made
+    by the caller is kept."""
+    rng = np.random.default_rng(14)
+    m = P.box_hexes(*n)
+    g, q = P.build_geometry(m, order), P.lqn(3, sn)
+    st = rng.uniform(0.3, 3.0, g.n_cells)
+    ctx = T.Context(g, q)
+    keep = (dev(st), dev(0.5 * st))
+    ctx.set_group(*keep)
+    sw = T.Sweep(ctx)
+    assert (sw.status()["kernel"] == T._lib.SWEEP_WAVE) == wave
+    op = O.Operator(g, q, st, 0.5 * st)
+    qv = rng.standard_normal(op.n)
+    ref = op.sweep(qv)
+    phi = dev(rng.standard_normal(ctx.n_nodes))
+
+    def check():
+        assert np.abs(sw.apply(dev(qv)).cpu().numpy() - ref).max() <= 1e-12 * np.abs(ref).max()
+        for dt, tol in ((torch.float64, 1e-12), (torch.float32, 1e-4)):
+            row = sw.apply_iso(phi, torch.empty(ctx.n_rows, dtype=dt, device="cuda"))
+            om = sw.apply_iso(phi, torch.empty(ctx.n_rows, dtype=dt, device="cuda"), ordinate_major=True)
+            om = om.reshape(q.n_angles, ctx.n_nodes).T.reshape(-1)
+            assert float((om - row).abs().max()) <= tol * float(row.abs().max())
+        assert sw.status()["timeouts"] == 0
+
+    check()
+    sw.set_kernel("tasks")
+    assert sw.status()["kernel"] == T._lib.SWEEP_TASKS
+    check()
+    sw.set_kernel("auto")
+    assert (sw.status()["kernel"] == T._lib.SWEEP_WAVE) == wave
+    check()
+    if wave:
+        sw.set_kernel("wave")
+        with pytest.raises(T._lib.UboltError):
+            sw.apply_iso(phi, torch.empty(ctx.n_rows, dtype=torch.float64, device="cuda"), ordinate_major=True)
+    # A whole solve and its adjoint, with the wave kernel's rows
+    b = dev(rng.uniform(0.1, 1.0, op.n))
+    for solve, mult in (("solve", T.TransportOperator(ctx).mult), ("solve_adjoint", T.TransportOperator(ctx).mult_transpose)):
+        x, s = getattr(T.TransportSolver(ctx, rtol=1e-10), solve)(b)
+        assert float(torch.linalg.norm(b - mult(x))) <= 1.01e-10 * float(torch.linalg.norm(b))
+    ctx.close()

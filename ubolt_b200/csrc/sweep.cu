@@ -76,12 +76,29 @@ constexpr int64_t kFewCellOrdinates = (int64_t)1 << 20;
 //    200^2 quads             64: 234 / 221    256: 225 / 212
 //    20^3 cubes of tets      48: 386 / 351    192: 213 / 196
 //    40^3 hexes              64: 150 / 136    128: 129 / 115    256: 155 / 125
+// A mesh of one patch has no task that waits on another (125 hexahedra DG1 S8
+// 24 -> 20; 162 tetrahedra without a factor store 36 -> 45, a patch of 48 36).
 static int DefaultPatch(const ubolt_ctx *ctx)
 {
+   if (ctx->n_cells <= 128) return 128;
    const bool tets = ctx->dim == 3 && ctx->F == 4;
    if (ctx->nb == 1) return ctx->dim == 2 ? 256 : tets ? 192 : 128;
    if (ctx->dim == 3) return tets ? 48 : 64;
    return ctx->n_cells * (int64_t)ctx->A <= kFewCellOrdinates ? 128 : 64;
+}
+
+// Where AUTO takes the wave kernel. One block per ordinate leaves most of the
+// device idle, and the task kernel was faster on the meshes measured (FP64,
+// us, wave and tasks: 64^2 quads DG0 S4 68 / 41, 32^2 37 / 23, 24^2 triangles DG1
+// S8 84 / 38, 16^3 hexes DG1 S2 72 / 53, 256^2 triangles DG1 S8 2220 / 703), but
+// for small DG0 boxes of hexahedra, whose levels are many cells of one value and
+// few: 10^3 S2 / S4 / S8 24 / 24 / 25 and 30 / 32 / 36, 16 x 15 x 17 S2 34 and 43, S4
+// 35 and 47; 20^3 S2 50 and 45. A whole solve there 530 / 542 / 541 and 588 / 598 /
+// 688 us at 10^3, 634 and 670 at 16 x 15 x 17, 786 and 691 at 20^3
+static bool WaveByDefault(const ubolt_ctx *ctx)
+{
+   return ctx->dim == 3 && ctx->F == 6 && ctx->nb == 1 && ctx->n_cells <= 4096 &&
+          ctx->n_cells * (int64_t)ctx->A <= (int64_t)1 << 17;
 }
 
 namespace ubolt {
@@ -119,7 +136,7 @@ struct ubolt_sweep_plan {
    // graph is acyclic and a level fits a block: wave[which].smem > 0 where
    // precision `which` (0 FP64, 1 FP32) can run it. fac_wave[which]: the
    // store reserved for that precision is in wave order (the wave kernel runs)
-   bool wave_tried = false, wave_ok = false;  // built when the wave kernel is asked for
+   bool wave_tried = false, wave_ok = false;  // built where the wave kernel is asked for or AUTO takes it
    int wave_threads = 256;
    int64_t wave_levels = 0;
    ubolt::WaveDev wave[2];
@@ -949,7 +966,7 @@ int BuildSweepPlan(ubolt_ctx *ctx, int patch_size)
       plan->fac_limit = ctx->sweep->fac_limit;
       plan->kernel_mode = ctx->sweep->kernel_mode;
    }
-   if (plan->kernel_mode == UBOLT_SWEEP_WAVE) {
+   if (plan->kernel_mode == UBOLT_SWEEP_WAVE || (plan->kernel_mode == UBOLT_SWEEP_AUTO && WaveByDefault(ctx))) {
       if ((rc = BuildWavePlan(ctx, plan))) { delete plan; return rc; }
       if (!plan->wave_ok) plan->kernel_mode = UBOLT_SWEEP_AUTO;
    }
@@ -1084,13 +1101,10 @@ static int ReserveFactors(ubolt_ctx *ctx, int64_t limit)
    }
    int64_t left = limit;
    for (int which : {1, 0}) {
-      // The wave kernel's store is in wave order. It runs where it is asked
-      // for: one block per ordinate leaves most of the device idle, and the
-      // task kernel was faster on every mesh measured (FP64, us, wave and
-      // tasks: 64^2 quads DG0 S4 68 / 41, 32^2 37 / 23, 24^2 triangles DG1 S8
-      // 84 / 38, 16^3 hexes DG1 S2 72 / 53, 8^3 hexes DG1 S4 27 / 25, 256^2
-      // triangles DG1 S8 2220 / 703)
-      const bool wave = pl->wave[which].smem > 0 && pl->kernel_mode == UBOLT_SWEEP_WAVE;
+      // The wave kernel's store is in wave order
+      const bool wave = pl->wave[which].smem > 0 &&
+                        (pl->kernel_mode == UBOLT_SWEEP_WAVE ||
+                         (pl->kernel_mode == UBOLT_SWEEP_AUTO && WaveByDefault(ctx)));
       pl->fac_wave[which] = false;
       const int64_t bytes = wave ? pl->wave_bytes[which] : FactorBytes(ctx, pl, which ? 4 : 8);
       if (bytes > left) continue;
@@ -1161,8 +1175,12 @@ static int LaunchSweep(ubolt_ctx *ctx, const T *q, T *psi, cudaStream_t st, cons
 {
    ubolt_sweep_plan *pl = ctx->sweep;
    const int which = sizeof(T) == 8 ? 0 : 1;
-   const T *fac = EnsureFactors<T, NB, F>(ctx, st);
-   if (pl->fac_wave[which]) {
+   // What the wave kernel cannot do the task kernel does where the
+   // choice is automatic, its factors formed as it goes: the store is the wave's
+   const bool not_wave = ordinate_major || q_om || (affine && affine->aff_inv_volume);
+   const bool wave = pl->fac_wave[which] && !(not_wave && pl->kernel_mode == UBOLT_SWEEP_AUTO);
+   const T *fac = pl->fac_wave[which] && !wave ? nullptr : EnsureFactors<T, NB, F>(ctx, st);
+   if (wave) {
       // One block per ordinate over the store in wave order (no sentinel fill)
       if (!fac) return UBOLT_ERR_CUDA;  // the failed launch set the message
       if (ordinate_major) return SetError(UBOLT_ERR_STATE, "the wave sweep writes the row layout only");
@@ -1344,7 +1362,8 @@ extern "C" int ubolt_sweep_set_kernel(ubolt_ctx *ctx, int kernel)
    if (kernel < UBOLT_SWEEP_AUTO || kernel > UBOLT_SWEEP_WAVE) return SetError(UBOLT_ERR_ARG, "sweep kernel %d", kernel);
    if (!ctx->sweep && (rc = BuildSweepPlan(ctx, 0))) return rc;
    ubolt_sweep_plan *pl = ctx->sweep;
-   if (kernel == UBOLT_SWEEP_WAVE && (rc = BuildWavePlan(ctx, pl))) return rc;
+   if ((kernel == UBOLT_SWEEP_WAVE || (kernel == UBOLT_SWEEP_AUTO && WaveByDefault(ctx))) && (rc = BuildWavePlan(ctx, pl)))
+      return rc;
    if (kernel == UBOLT_SWEEP_WAVE && !pl->wave_ok)
       return SetError(UBOLT_ERR_STATE, "the wave sweep does not apply here (an upwind cycle, or a level or front too "
                                        "large for one block)");
@@ -1370,7 +1389,8 @@ static int SweepIso(ubolt_ctx *ctx, const double *phi, const T *u, T *psi, int o
    int rc = CheckReady(ctx, true);
    if (rc) return rc;
    if (!phi || !psi) return SetError(UBOLT_ERR_ARG, "sweep_iso: NULL array");
-   if (ordinate_major && !SweepWritesOrdinateMajor<T>(ctx))
+   if (!ctx->sweep && (rc = BuildSweepPlan(ctx, 0))) return rc;
+   if (ordinate_major && ctx->sweep->kernel_mode == UBOLT_SWEEP_WAVE && !SweepWritesOrdinateMajor<T>(ctx))
       return SetError(UBOLT_ERR_STATE, "sweep_iso: the wave kernel runs here, and it writes the row layout only");
    return SweepAffine<T>(ctx, nullptr, nullptr, phi, nullptr, u, psi, stream, ordinate_major != 0, false);
 }
