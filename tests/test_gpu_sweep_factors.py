@@ -48,3 +48,58 @@ def test_store_equals_factors_formed_in_the_sweep(case):
     assert all(torch.equal(a, b) for a, b in zip(stored, formed))
     assert sw.status()["timeouts"] == 0 and bool(torch.isfinite(stored[0]).all())
     ctx.close()
+
+
+@pytest.mark.parametrize("case", ["dg0", "few_rows", "scratch"])
+def test_scratch_vector_is_held_only_where_a_sweep_uses_it(case):
+    """Row vectors pass through a scratch vector from two rows per cell and 8 MB
+    on; nothing is held for others. A limit below either store leaves it alone."""
+    m = P.box_quads(*{"dg0": (600, 500), "few_rows": (160, 150), "scratch": (256, 250)}[case])
+    g, q = P.build_geometry(m, 0 if case == "dg0" else 1), P.lqn(2, 4)
+    ctx = T.Context(g, q)
+    sw = T.Sweep(ctx, factor_limit=0)
+    vec = 8 * ctx.n_rows
+    before = torch.cuda.mem_get_info()[0]
+    sw.set_factor_limit(vec)
+    assert sw.status()["factor_bytes"] == 0
+    held = before - torch.cuda.mem_get_info()[0]
+    # (the allocator's pages: 2 MB)
+    assert abs(held - (vec if case == "scratch" else 0)) <= 4 << 20
+    assert vec > (8 << 20 if case != "few_rows" else 6 << 20)
+    ctx.close()
+
+
+SCRATCH = {
+    # nb > 1 and 8 MB (FP32) and more, more than 64 ordinates in equal parts (80: two
+    # of 40, 180: three of 60) and in uneven ones (288: four of 58 and one of 56), node
+    # counts that are no multiple of 64
+    "quad_s12": (lambda r: P.box_quads(97, 89, jitter=0.2, rng=r), 12),
+    "tri_s18": (lambda r: P.box_tris(51, 47, jitter=0.2, rng=r), 18),
+    "hex_s16": (lambda r: P.box_hexes(13, 13, 13), 16),
+    "tet_s8": (lambda r: P.box_tets(11, 11, 11, jitter=0.1, rng=r), 8),
+    "hex_s8": (lambda r: P.box_hexes(21, 19, 17), 8),
+    "hex_s10": (lambda r: P.box_hexes(19, 17, 15), 10),
+}
+
+
+@pytest.mark.parametrize("case", SCRATCH)
+def test_row_sweeps_through_the_scratch_vector(case):
+    """Bit for bit the direct sweep of rows (no store and no scratch vector)."""
+    make, sn = SCRATCH[case]
+    rng = np.random.default_rng(32)
+    m = make(rng)
+    g, q = P.build_geometry(m, 1), P.lqn(m.dim, sn)
+    st = rng.uniform(0.3, 3.0, g.n_cells)
+    ctx = T.Context(g, q)
+    assert 4 * ctx.n_rows >= 8 << 20 and ctx.n_nodes % 64 != 0
+    keep = (torch.tensor(st, device="cuda"), torch.tensor(0.5 * st, device="cuda"))
+    ctx.set_group(*keep)
+    sw = T.Sweep(ctx)
+    x = torch.tensor(rng.standard_normal(ctx.n_rows), device="cuda")
+    keep_x = x.clone()
+    through = [sw.apply(x), sw.apply(x.float())]
+    sw.set_factor_limit(0)
+    direct = [sw.apply(x), sw.apply(x.float())]
+    assert all(torch.equal(a, b) for a, b in zip(through, direct)) and torch.equal(x, keep_x)
+    assert sw.status()["timeouts"] == 0 and bool(torch.isfinite(direct[0]).all())
+    ctx.close()

@@ -1118,7 +1118,8 @@ static int ReserveFactors(ubolt_ctx *ctx, int64_t limit)
       left -= bytes;
    }
    const int64_t vec = ctx->n_rows * (int64_t)sizeof(double);
-   if (vec <= left && !(pl->fac_wave[0] && pl->fac_wave[1])) {
+   // (only where a sweep between row vectors goes through it, see LaunchSweep)
+   if (ctx->nb > 1 && vec >= (int64_t)kViaBytes && vec <= left && !(pl->fac_wave[0] && pl->fac_wave[1])) {
       if (cudaMalloc(&pl->scratch, (size_t)vec) != cudaSuccess) {
          cudaGetLastError();
          pl->scratch = nullptr;
