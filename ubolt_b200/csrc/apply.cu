@@ -99,6 +99,18 @@ constexpr int ApplyMinBlocks() { return (NB == 4 && AP > 1) ? 2 : 3; }
 template <int NB, int F, int AP>
 constexpr bool ApplyRounds() { return UpSlots<NB, F>() < F && AP > 1; }
 
+// True where a thread reads its cell's class and face codes before the block's
+// copies, whose order among themselves makes a code read between two of them
+// wait alone (256^2 DG1 triangles FP64 134 -> 131 us, DG0 unscattered S16 165 ->
+// 156). Two FP64 kernels are faster with the rows' copies issued first: DG0
+// triangles with the scatter (256^2 S8 70 and 66 us, S16 247 and 236) and DG1
+// quadrilaterals without (301 x 257 S4 47 and 45)
+template <typename T, int NB, int F, bool SCATTER, bool REV>
+constexpr bool ApplyCodesFirst()
+{
+   return !(sizeof(T) == 8 && ((NB == 1 && F == 3 && SCATTER && !REV) || (NB == 3 && F == 4 && !SCATTER)));
+}
+
 // REV: the transpose (L - S)^T = L^T - S^T, L^T as the reversed-angle
 // operator. (V L)^T = P (V L) P (V the cell volume on every row, P the swap
 // of each ordinate with its opposite) gives L^T x = P V L (P V^{-1} x): the
@@ -118,6 +130,7 @@ __global__ void __launch_bounds__(256, ApplyMinBlocks<T, NB, AP>()) ApplyKernel(
    constexpr int XS = UpSlots<NB, F>();
    constexpr bool kRing = XS < F;
    constexpr bool kRounds = ApplyRounds<NB, F, AP>();
+   constexpr bool kCodesFirst = ApplyCodesFirst<T, NB, F, SCATTER, REV>();
    extern __shared__ __align__(16) unsigned char smem_raw[];
    const int A = g.A, QA = A / AP;
    T *recs = reinterpret_cast<T *>(smem_raw);
@@ -145,14 +158,13 @@ __global__ void __launch_bounds__(256, ApplyMinBlocks<T, NB, AP>()) ApplyKernel(
       const int kc = (int)min((int64_t)K, g.n_cells - c0);
       const bool live = k < kc;
       int32_t code[F], cls = 0;
-      // Read together, before any copy: the copies are ordered among themselves,
-      // so a code read between two of them would wait alone (256^2 triangles FP64
-      // 134 -> 131 us)
-      if (live) {
-         cls = g.cls[c];
+      // Read together, before any copy, where that is faster (ApplyCodesFirst)
+      if constexpr (kCodesFirst)
+         if (live) {
+            cls = g.cls[c];
 #pragma unroll
-         for (int f = 0; f < F; f++) code[f] = g.code[c * F + f];
-      }
+            for (int f = 0; f < F; f++) code[f] = g.code[c * F + f];
+         }
 
       // Stage: the block's own rows (one contiguous range), each cell's class
       // record and this thread's upwind runs, all in flight at once (with the
@@ -165,6 +177,7 @@ __global__ void __launch_bounds__(256, ApplyMinBlocks<T, NB, AP>()) ApplyKernel(
          for (int u = t; u < nu; u += blockDim.x) CpAsyncRun<CU>(reinterpret_cast<unsigned char *>(xs) + u * CU, src + u * CU);
       }
       if (live) {
+         if constexpr (!kCodesFirst) cls = g.cls[c];
          const T *rec = g.rec + (int64_t)cls * L.size;
          for (int u = q; u < RU; u += QA) CpAsync<16>(recs + k * L.size + u * (16 / (int)sizeof(T)), rec + u * (16 / (int)sizeof(T)));
          if constexpr (kRing) CpAsyncCommit();
@@ -172,7 +185,7 @@ __global__ void __launch_bounds__(256, ApplyMinBlocks<T, NB, AP>()) ApplyKernel(
          if constexpr (REV) vc = g.volume[c];
 #pragma unroll
          for (int f = 0; f < F; f++) {
-            const int32_t cf = code[f];
+            const int32_t cf = kCodesFirst ? code[f] : g.code[c * F + f];
             if (FaceInterior(cf)) {
                fcode |= 8u << (4 * f);
                if constexpr (REV) rat[f * (int)blockDim.x + t] = vc * g.inv_vol[g.cls[cf]];
