@@ -95,21 +95,22 @@ constexpr int64_t kSpmvRowCells = 49152;
 // A cell's matrix in shared memory, an odd number of values apart (no bank conflicts)
 __host__ __device__ constexpr int KeptStride(int F, int NB) { return (F + 1) * NB * NB | 1; }
 
+// A cell's neighbours. A face without one has a zero block: the cell itself
+// stands for it, so that no lane branches on its own
 template <int F>
 __device__ __forceinline__ void CellNeighbours(int64_t c, const int32_t *__restrict__ code, int32_t (&nbr)[F])
 {
 #pragma unroll
-   for (int f = 0; f < F; f++) nbr[f] = code[c * F + f];
+   for (int f = 0; f < F; f++) {
+      const int32_t n = code[c * F + f];
+      nbr[f] = n < 0 ? (int32_t)c : n;
+   }
 }
 
-// sum_{f, j} D(i; f, j) x(f, j) over cell c's neighbours and itself for its NB
-// rows: x(cell, j) given by `at`, element k of the cell's matrix by `val`. A
-// face without a neighbour has a zero block: it reads the cell itself, so that
-// no lane branches on its own, and takes zero for it (an infinite value times
-// a zero block would not be nothing)
+// sum_{f, j} D(i; f, j) x(f, j) over a cell's neighbours and itself for its NB
+// rows: x(f, j) given by `at`, element k of the cell's matrix by `val`
 template <int NB, int F, typename Val, typename At>
-__device__ __forceinline__ void CellRows(int64_t c, const int32_t (&nbr)[F], Val val, const double (&own)[NB], At at,
-                                         double (&s)[NB])
+__device__ __forceinline__ void CellRows(Val val, const double (&own)[NB], At at, double (&s)[NB])
 {
 #pragma unroll
    for (int i = 0; i < NB; i++) s[i] = 0.0;
@@ -117,10 +118,7 @@ __device__ __forceinline__ void CellRows(int64_t c, const int32_t (&nbr)[F], Val
    for (int f = 0; f < F; f++) {
       double x[NB];
 #pragma unroll
-      for (int j = 0; j < NB; j++) {
-         const double v = at(nbr[f] < 0 ? (int32_t)c : nbr[f], j);
-         x[j] = nbr[f] < 0 ? 0.0 : v;
-      }
+      for (int j = 0; j < NB; j++) x[j] = at(f, j);
 #pragma unroll
       for (int i = 0; i < NB; i++)
 #pragma unroll
@@ -132,7 +130,9 @@ __device__ __forceinline__ void CellRows(int64_t c, const int32_t (&nbr)[F], Val
       for (int j = 0; j < NB; j++) s[i] += val((F * NB + i) * NB + j) * own[j];
 }
 
-// v = D u over the block-ELL rows, one thread per cell
+// v = D u over the block-ELL rows, one thread per cell. A face without a
+// neighbour counts as zero, not as its zero block times the value read for it: that
+// value may be infinite
 template <int NB, int F>
 __global__ void __launch_bounds__(128) DsaSpmvKernel(int64_t nc, const int32_t *__restrict__ code,
                                                      const double *__restrict__ val, const double *__restrict__ u,
@@ -144,9 +144,14 @@ __global__ void __launch_bounds__(128) DsaSpmvKernel(int64_t nc, const int32_t *
 #pragma unroll
    for (int j = 0; j < NB; j++) own[j] = u[c * NB + j];
    int32_t nbr[F];
-   CellNeighbours<F>(c, code, nbr);
-   CellRows<NB, F>(c, nbr, [&](int k) { return __ldg(val + (int64_t)k * nc + c); }, own,
-                   [&](int32_t n, int j) { return u[(int64_t)n * NB + j]; }, s);
+#pragma unroll
+   for (int f = 0; f < F; f++) nbr[f] = code[c * F + f];
+   CellRows<NB, F>([&](int k) { return __ldg(val + (int64_t)k * nc + c); }, own,
+                   [&](int f, int j) {
+                      const double x = u[(nbr[f] < 0 ? c : (int64_t)nbr[f]) * NB + j];
+                      return nbr[f] < 0 ? 0.0 : x;
+                   },
+                   s);
 #pragma unroll
    for (int i = 0; i < NB; i++) v[c * NB + i] = s[i];
 }
@@ -162,7 +167,8 @@ __global__ void __launch_bounds__(128) DsaSpmvRowKernel(int64_t nc, const int32_
    const int i = blockIdx.y;
    if (c >= nc) return;
    int32_t nbr[F];
-   CellNeighbours<F>(c, code, nbr);
+#pragma unroll
+   for (int f = 0; f < F; f++) nbr[f] = code[c * F + f];
    double d[F + 1][NB], x[F + 1][NB];
 #pragma unroll
    for (int f = 0; f <= F; f++)
@@ -276,8 +282,9 @@ struct DsaPcgArgs {
 // barrier: each block leaves its share in slots[step parity][block], arrives on
 // the counter and waits for all blocks; then the shares are added in a fixed
 // order. Bounded; false (in every thread of the block): gave up. About 1.3 us
-// with 296 blocks and one thread of each polling the counter; every block
-// polling every other's slot instead took 6 us.
+// with one thread of a block polling the counter, measured with 296 blocks (148
+// run, 296 for many vertices); every block polling every other's slot instead
+// took 6 us.
 __device__ __forceinline__ bool GridSum(double d, const DsaPcgArgs &a, unsigned step, double *sum)
 {
    constexpr int kWarps = kPcgThreads / 32;
@@ -394,9 +401,9 @@ __global__ void __launch_bounds__(kPcgThreads, PcgBlocksPerSm(CSR, OWN)) DsaPcgK
             for (int64_t k = a.rp[c]; k < a.rp[c + 1]; k++) q[0] += __ldg(a.val + k) * direction(a.col[k]);
          } else {
             if constexpr (!OWN) CellNeighbours<F>(c, a.code, nbr);
-            auto at = [&](int32_t n, int j) { return direction((int64_t)n * NB + j); };
-            if constexpr (KEEP) CellRows<NB, F>(c, nbr, [&](int k) { return mine[k]; }, p, at, q);
-            else CellRows<NB, F>(c, nbr, [&](int k) { return __ldg(a.val + (int64_t)k * a.n + c); }, p, at, q);
+            auto at = [&](int f, int j) { return direction((int64_t)nbr[f] * NB + j); };
+            if constexpr (KEEP) CellRows<NB, F>([&](int k) { return mine[k]; }, p, at, q);
+            else CellRows<NB, F>([&](int k) { return __ldg(a.val + (int64_t)k * a.n + c); }, p, at, q);
          }
 #pragma unroll
          for (int i = 0; i < NB; i++) {

@@ -37,9 +37,9 @@
 // level's arithmetic), and a wait asks for what the next levels wait for as
 // well. Per sweep with an isotropic source and psi ordinate-major, before (a
 // lane per cell, each level polling for itself) and now, FP64 / FP32: 256^2
-// triangles 942 / 791 -> 595 / 486 us, 200^2 quadrilaterals 635 / 555 -> 316 /
-// 267, 20^3 cubes of Kuhn tetrahedra 1447 / 1159 -> 982 / 678, 40^3 hexahedra
-// 1186 / 684 -> 593 / 402.
+// triangles 945 / 795 -> 593 / 489 us, 200^2 quadrilaterals 643 / 562 -> 308 /
+// 275, 20^3 cubes of Kuhn tetrahedra 1453 / 1166 -> 905 / 496, 40^3 hexahedra
+// 1188 / 687 -> 605 / 400.
 #include "ctx.h"
 #include "sweep_plan.h"
 #include "wave.h"
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 && NB == 4 ? 1 : 2) Factor
 
 // Blocks of two warps the registers should leave room for per SM: eight (at
 // most 128 registers), ten for FP32 tetrahedra, whose small tasks are bound by
-// their number in flight (678 against 780 us per sweep of 20^3 cubes; the
+// their number in flight (496 against 537 us per sweep of 20^3 cubes; the
 // other shapes measured the same or slower), and no cap where the blocks would
 // spill heavily and shared memory holds fewer anyway
 template <typename T, int NB, int S, int KU>
@@ -1207,7 +1207,8 @@ static int LaunchSweep(ubolt_ctx *ctx, const T *q, T *psi, cudaStream_t st, cons
    const size_t slice = (size_t)SweepSlice(pl->P, pl->slots, F, NB, pl->n_loc, pl->n_ghost, (int)sizeof(T), fac != nullptr).bytes;
    constexpr int S0 = F == 6 ? 3 : 2;
    // Two positions per lane in a prologue where the tasks hold more than a
-   // warp's worth, one where they are small (jittered tetrahedra: 8 cells of 24)
+   // warp's worth, one where they are small (jittered tetrahedra, whose patches'
+   // cells are split over several tasks)
    const bool wide = ctx->n_cells * (int64_t)ctx->A > 24 * pl->n_tasks;
    auto kern = pl->slots == S0 ? (fac ? (wide ? SweepKernel<T, NB, F, S0, 2, true> : SweepKernel<T, NB, F, S0, 1, true>)
                                       : (wide ? SweepKernel<T, NB, F, S0, 2, false> : SweepKernel<T, NB, F, S0, 1, false>))
